@@ -990,22 +990,28 @@ const void *any_walk_kernel(bool fp64, bool adj, int damping, bool pot, bool sta
 constexpr size_t kLargestWarpSmem =
     sizeof(WarpSmem<true>) > sizeof(WarpSmem<false>) ? sizeof(WarpSmem<true>) : sizeof(WarpSmem<false>);
 
+// The grid is sized by the forward walk's instances. The adjoint's FP64 ones take
+// more registers (138-152 against 94-96): fewer of their blocks are resident, and
+// the rest start as those end and find the work counter drained (the walk waits on
+// nothing). Sizing every launch by the largest instance kept the FP64 forward walk
+// at 3 resident blocks of the 5 that fit: 1.295 -> 1.161 ms (sphere of 60,001,
+// damped), 2.27 -> 1.76 ms (sphere of 200,000).
 cudaError_t walk_max_blocks_per_sm(bool fp64, unsigned warps, int *out) {
     const size_t smem = (fp64 ? sizeof(WarpSmem<true>) : sizeof(WarpSmem<false>)) * warps;
     int minblocks = 1 << 30;
-    for (int adj = 0; adj < 2; adj++)
-        for (int damp = 0; damp < 2; damp++)
-            for (int pot = 0; pot < 2 - adj; pot++)
-                for (int stats = 0; stats < 2 - adj; stats++) {
-                    const void *k = any_walk_kernel(fp64, adj, damp, pot, stats);
-                    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                         (int)(kLargestWarpSmem * kWalkMaxWarps));
-                    if (e != cudaSuccess) return e;
-                    int nb = 0;
-                    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k, (int)warps * 32, smem);
-                    if (e != cudaSuccess) return e;
-                    minblocks = nb < minblocks ? nb : minblocks;
-                }
+    for (int q = 0; q < 16; q++) {
+        const bool adj = q & 1, damp = q & 2, pot = q & 4, stats = q & 8;
+        if (adj && (pot || stats)) continue;
+        const void *k = any_walk_kernel(fp64, adj, damp, pot, stats);
+        cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             (int)(kLargestWarpSmem * kWalkMaxWarps));
+        if (e != cudaSuccess) return e;
+        if (adj) continue;
+        int nb = 0;
+        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k, (int)warps * 32, smem);
+        if (e != cudaSuccess) return e;
+        minblocks = nb < minblocks ? nb : minblocks;
+    }
     *out = minblocks;
     return cudaSuccess;
 }

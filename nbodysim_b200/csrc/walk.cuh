@@ -60,7 +60,7 @@ struct WalkLaunch {
 };
 // blocks_per_sm = 0: as many as fit. Returns the shape for that block size.
 cudaError_t walk_launch_shape(bool fp64, int device, unsigned warps, unsigned blocks_per_sm, WalkLaunch *out);
-// Resident blocks per SM that fit for `warps` per block (all walk variants).
+// Resident blocks per SM that fit for `warps` per block (all forward instances).
 cudaError_t walk_max_blocks_per_sm(bool fp64, unsigned warps, int *out);
 cudaError_t launch_walk(const WalkArgs &a, bool fp64, const WalkLaunch &l, cudaStream_t st);
 

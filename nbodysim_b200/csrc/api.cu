@@ -1565,7 +1565,7 @@ int nbody_direct_forces(nbody_ctx *c, uint32_t m, const uint32_t *targets, int d
         for (uint32_t w = 0; w < m; w++)
             if (targets[w] >= c->n) return fail(NBODY_ERR_INVALID, "target index out of range%s");
     if (m == 0) return NBODY_OK;
-    const size_t need = align256(4 * (size_t)m) + align256(24 * (size_t)m);
+    const size_t need = align256(4 * (size_t)m) + align256(24 * (size_t)m) + direct_scratch_bytes(c->n, m);
     if (need > c->direct_bytes) {
         NB_CUDA(cudaStreamSynchronize(c->stream));
         if (c->direct_arena) NB_CUDA(cudaFree(c->direct_arena));
@@ -1581,8 +1581,11 @@ int nbody_direct_forces(nbody_ctx *c, uint32_t m, const uint32_t *targets, int d
     uint32_t *d_t = (uint32_t *)c->direct_arena;
     double *d_out = (double *)((char *)c->direct_arena + align256(4 * (size_t)m));
     if (targets) NB_CUDA(cudaMemcpyAsync(d_t, targets, 4 * (size_t)m, cudaMemcpyHostToDevice, c->stream));
-    NB_CUDA(launch_direct(c->pos, c->mass, c->n, damping, targets ? d_t : nullptr, m, d_out, c->stream));
-    c->launches++;
+    double *d_part = (double *)((char *)d_out + align256(24 * (size_t)m));
+    unsigned launches = 0;
+    NB_CUDA(launch_direct(c->pos, c->mass, c->n, damping, targets ? d_t : nullptr, m, d_out, d_part, c->stream,
+                          &launches));
+    c->launches += launches;
     NB_CUDA(cudaMemcpyAsync(acc_out, d_out, 24 * (size_t)m, cudaMemcpyDeviceToHost, c->stream));
     NB_CUDA(cudaStreamSynchronize(c->stream));
     return NBODY_OK;

@@ -677,8 +677,8 @@ int apply_collisions(nbody_ctx *c, unsigned *launches) {
     uint32_t np = 0;
     for (int attempt = 0; attempt < 2; attempt++) {
         NB_CUDA(merge_begin(c->mb, c->n, c->stream, launches));
-        NB_CUDA(collide_find(c->mb, tree_view(c), c->tb.oparent, c->p.theta, c->p.collision_range, c->stream,
-                             launches));
+        NB_CUDA(collide_find(c->mb, tree_view(c), c->tb.oparent, c->tb.leaf_oparent, c->p.theta,
+                             c->p.collision_range, c->stream, launches));
         if ((rc = read_counters(c))) return rc;
         np = c->hcounters[kMcPairs];
         if (np <= c->mb.pair_cap) break;

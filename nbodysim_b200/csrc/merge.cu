@@ -16,10 +16,9 @@
 // topmost branching node inside the cell is the reference's fold, bit for bit.
 //
 // Collisions: a particle records a pair with every leaf its walk accepts that
-// lies closer than the collision range. A separate walk per particle replays
-// the reference's FP64 opening test exactly, but only inside nodes that can
-// hold a leaf within range (every particle of a node lies in its cube, within
-// side * sqrt(3) of its centre of mass). Pairs become connected components
+// lies closer than the collision range. A separate search finds the leaves within
+// range and replays the reference's FP64 opening test exactly on their ancestors.
+// Pairs become connected components
 // (union-find, root = smallest user index). The reference merges the pairs in
 // the iteration order of an unordered_set, so its result for a group of three
 // or more depends on pointer hashes; here each component is folded in
@@ -144,73 +143,135 @@ __global__ void k_min_size(Tree t, const int32_t *__restrict__ oparent, const do
     atomicAdd(&m.counters[kMcGroups], 1u);
 }
 
-// One thread per particle (Morton order): a stackless walk (parent links) that
-// opens exactly what the reference opens, restricted to nodes that can hold a
-// leaf within range.
-__global__ void k_collide_find(Tree t, const int32_t *__restrict__ oparent, double theta, double range,
-                               MergeBufs m) {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= t.n || t.n < 2) return;
-    const double4 bi = t.body[i];
-    const double S = t.sc->root_side;
-    int node = 0;
-    bool enter = true;
-    for (uint32_t guard = 0; guard < 4 * t.n + 16; guard++) {
-        if (enter) {
-            const double4 nd = t.onode[node];
-            const int32_t meta = t.ometa[node];
-            const double side = S * exp2_neg(meta_level(meta));
-            const double d = exact_dist(nd.x, nd.y, nd.z, bi.x, bi.y, bi.z);
-            bool open = !(d > (range + side * 1.7320508075688772) * (1.0 + 1e-9));
-            if (open) open = __ddiv_rn(side, d) > theta;  // src/main.cpp:377
-            if (open) {
-                int first = -1;
-                const int nch = meta_nchild(meta);
-                for (int k = 0; k < nch; k++) {
-                    const int32_t ch = t.ochild[8 * node + k];
-                    if (ch >= 0) {
-                        if (first < 0) first = ch;
-                        continue;
-                    }
-                    const uint32_t j = ~(uint32_t)ch;
-                    if (j == i) continue;  // a particle's own leaf is never accepted
-                    const double4 bj = t.body[j];
-                    if (exact_dist(bj.x, bj.y, bj.z, bi.x, bi.y, bi.z) < range) {  // src/main.cpp:386
-                        const uint32_t ui = t.sidx[i], uj = t.sidx[j];
-                        const uint32_t slot = atomicAdd(&m.counters[kMcPairs], 1u);
-                        if (slot < m.pair_cap) m.pairs[slot] = make_uint2(min(ui, uj), max(ui, uj));
-                    }
-                }
-                if (first >= 0) {
-                    node = first;
-                    continue;
-                }
-            }
+// Collision search: one warp per 32 Morton-consecutive particles.
+//
+// Bound: instruction issue. A stackless walk per particle with the exact opening
+// test (FP64 square root and divide) at every node took 385 M warp instructions and
+// 1.62 ms on a cube of 60,000 (range 0.5); this search takes 0.124 ms. There, lanes of a warp sit in different
+// subtrees, and a node's test costs ~100 instructions. Here a lane takes one stacked
+// node or leaf and asks whether it can hold a particle within range of the group's
+// box (every particle of a node lies within side * sqrt(3) of its centre of mass);
+// what is left is asked of every particle of the group by squared distances (without
+// that, a group that straddles a large cell has a box full of nodes near no particle,
+// and the few such groups take 1.2 ms). The few pairs within range then climb the
+// leaf's ancestors with the exact opening test, which is what decides whether the
+// reference's walk reaches the leaf.
+constexpr int kFindWarps = 4;
+// The stack keeps room for a depth-first descent of one entry at a time (at most 7
+// more entries per level); tiles get narrower as it fills up to that reserve.
+constexpr int kFindReserve = 7 * (kMaxLevels + 1) + 8;
+constexpr int kFindStack = 1152;
+static_assert(kFindStack - kFindReserve >= 2 * 32 * 8, "room for full tiles above the reserve");
+
+// Whether the walk of the particle at b opens every ancestor of the leaf j (src/main.cpp:377).
+__device__ inline bool opens_to_leaf(const Tree &t, const int32_t *oparent, const int32_t *leaf_oparent, uint32_t j,
+                                     const double4 &b, double S, double theta, uint32_t *status) {
+    int p = leaf_oparent[j];
+    for (int hops = 0; p >= 0; hops++) {
+        if (hops > kMaxLevels + 1 || p >= (int)(t.n - 1)) {
+            atomicOr(status, kMergeStatusTree);
+            return false;
         }
-        // the next internal sibling, climbing while a node has none
-        if (node == 0) return;
-        const int32_t par = oparent[node];
-        if (par < 0) break;
-        const int nch = meta_nchild(t.ometa[par]);
-        int k = 0;
-        while (k < nch && t.ochild[8 * par + k] != node) k++;
-        int nxt = -1;
-        for (k++; k < nch; k++) {
-            const int32_t ch = t.ochild[8 * par + k];
-            if (ch >= 0) {
-                nxt = ch;
-                break;
-            }
-        }
-        if (nxt >= 0) {
-            node = nxt;
-            enter = true;
-        } else {
-            node = par;
-            enter = false;
-        }
+        const double4 nd = t.onode[p];
+        const double side = S * exp2_neg(meta_level(t.ometa[p]));
+        if (!(__ddiv_rn(side, exact_dist(nd.x, nd.y, nd.z, b.x, b.y, b.z)) > theta)) return false;
+        p = oparent[p];
     }
-    atomicOr(&m.counters[kMcStatus], kMergeStatusTree);
+    return true;
+}
+
+__global__ void __launch_bounds__(kFindWarps * 32)
+    k_collide_find(Tree t, const int32_t *__restrict__ oparent, const int32_t *__restrict__ leaf_oparent, double theta,
+                   double range, MergeBufs m) {
+    __shared__ int32_t s_stack[kFindWarps][kFindStack];
+    __shared__ double4 s_tile[kFindWarps][32];  // centre of mass or body, squared reach
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const uint32_t g0 = 32 * (blockIdx.x * kFindWarps + wid);
+    if (g0 >= t.n || t.n < 2) return;
+    int32_t *stack = s_stack[wid];
+    const unsigned FULL = 0xffffffffu;
+    const uint32_t lt = (1u << lane) - 1u;
+    const uint32_t i = g0 + lane;
+    const bool valid = i < t.n;
+    const double4 bi = t.body[valid ? i : g0];
+    const double lox = warp_min(bi.x), hix = warp_max(bi.x), loy = warp_min(bi.y), hiy = warp_max(bi.y),
+                 loz = warp_min(bi.z), hiz = warp_max(bi.z);
+    const double S = t.sc->root_side;
+    int top = 1;
+    if (lane == 0) stack[0] = 0;
+    __syncwarp();
+    uint64_t seen = 0;
+    while (top > 0) {
+        const int take = max(1, min(min(top, 32), (kFindStack - kFindReserve - top) / 8));
+        top -= take;
+        seen += take;
+        if (seen > 4ull * t.n + 64) {  // more entries than a well-formed octree holds
+            if (lane == 0) atomicOr(&m.counters[kMcStatus], kMergeStatusTree);
+            return;
+        }
+        int32_t ref = -1;
+        int nch = 0;
+        int4 c0 = make_int4(0, 0, 0, 0), c1 = c0;
+        bool near = false;
+        double4 q = make_double4(0.0, 0.0, 0.0, 0.0);
+        if (lane < take) {
+            ref = stack[top + lane];
+            double reach = range;
+            if (ref >= 0) {
+                q = t.onode[ref];
+                const int32_t meta = t.ometa[ref];
+                nch = meta_nchild(meta);
+                const int4 *cp = reinterpret_cast<const int4 *>(t.ochild + 8 * (size_t)ref);
+                c0 = cp[0];
+                c1 = cp[1];
+                reach = range + S * exp2_neg(meta_level(meta)) * 1.7320508075688772;
+            } else {
+                q = t.body[~ref];
+            }
+            const double reach2 = reach * reach * (1.0 + 4e-9);
+            const double dx = fmax(fmax(lox - q.x, q.x - hix), 0.0), dy = fmax(fmax(loy - q.y, q.y - hiy), 0.0),
+                         dz = fmax(fmax(loz - q.z, q.z - hiz), 0.0);
+            near = !(dx * dx + dy * dy + dz * dz > reach2);
+            s_tile[wid][lane] = make_double4(q.x, q.y, q.z, reach2);
+        }
+        __syncwarp();
+        const uint32_t leaves = __ballot_sync(FULL, ref < 0);
+        for (uint32_t left = __ballot_sync(FULL, near); left; left &= left - 1) {
+            const int k = __ffs(left) - 1;
+            const double4 e = s_tile[wid][k];
+            const double dx = e.x - bi.x, dy = e.y - bi.y, dz = e.z - bi.z;
+            const bool in = valid && !(dx * dx + dy * dy + dz * dz > e.w);
+            if (!((leaves >> k) & 1u)) {
+                const uint32_t any = __ballot_sync(FULL, in);
+                if (lane == k) near = any != 0u;
+                continue;
+            }
+            const uint32_t j = ~(uint32_t)__shfl_sync(FULL, ref, k);
+            if (!in || j == i) continue;  // a particle's own leaf is never accepted
+            if (!(exact_dist(e.x, e.y, e.z, bi.x, bi.y, bi.z) < range)) continue;  // src/main.cpp:386
+            if (!opens_to_leaf(t, oparent, leaf_oparent, j, bi, S, theta, &m.counters[kMcStatus])) continue;
+            const uint32_t ui = t.sidx[i], uj = t.sidx[j];
+            const uint32_t slot = atomicAdd(&m.counters[kMcPairs], 1u);
+            if (slot < m.pair_cap) m.pairs[slot] = make_uint2(min(ui, uj), max(ui, uj));
+        }
+        __syncwarp();
+        // children of the nodes in reach
+        const int myn = near && ref >= 0 ? nch : 0;
+        const uint32_t q0 = __ballot_sync(FULL, myn & 1), q1 = __ballot_sync(FULL, myn & 2),
+                       q2 = __ballot_sync(FULL, myn & 4), q3 = __ballot_sync(FULL, myn & 8);
+        const int pre = __popc(q0 & lt) + 2 * __popc(q1 & lt) + 4 * __popc(q2 & lt) + 8 * __popc(q3 & lt);
+        int32_t *dst = stack + top + pre;
+        if (myn > 0) dst[0] = c0.x;
+        if (myn > 1) dst[1] = c0.y;
+        if (myn > 2) dst[2] = c0.z;
+        if (myn > 3) dst[3] = c0.w;
+        if (myn > 4) dst[4] = c1.x;
+        if (myn > 5) dst[5] = c1.y;
+        if (myn > 6) dst[6] = c1.z;
+        if (myn > 7) dst[7] = c1.w;
+        top += __popc(q0) + 2 * __popc(q1) + 4 * __popc(q2) + 8 * __popc(q3);
+        __syncwarp();
+    }
 }
 
 // Root of x. Links only ever point to a smaller index, so the chase ends
@@ -316,10 +377,10 @@ cudaError_t merge_min_size(const MergeBufs &m, const Tree &t, const int32_t *opa
     return cudaGetLastError();
 }
 
-cudaError_t collide_find(const MergeBufs &m, const Tree &t, const int32_t *oparent, double theta, double range,
-                         cudaStream_t st, unsigned *launches) {
+cudaError_t collide_find(const MergeBufs &m, const Tree &t, const int32_t *oparent, const int32_t *leaf_oparent,
+                         double theta, double range, cudaStream_t st, unsigned *launches) {
     if (t.n < 2) return cudaSuccess;
-    k_collide_find<<<blocks_for(t.n, 128), 128, 0, st>>>(t, oparent, theta, range, m);
+    k_collide_find<<<blocks_for(t.n, kFindWarps * 32), kFindWarps * 32, 0, st>>>(t, oparent, leaf_oparent, theta, range, m);
     *launches += 1;
     return cudaGetLastError();
 }

@@ -48,10 +48,10 @@ cudaError_t merge_min_size(const MergeBufs &m, const Tree &t, const int32_t *opa
                            double min_size, cudaStream_t st, unsigned *launches);
 
 // The collision capture of barnes_hut_thread (src/main.cpp:386-396): pairs
-// (particle, accepted leaf) closer than `range`, found by a walk that replays
-// the reference's opening decisions only where a leaf can be within range.
-cudaError_t collide_find(const MergeBufs &m, const Tree &t, const int32_t *oparent, double theta, double range,
-                         cudaStream_t st, unsigned *launches);
+// (particle, accepted leaf) closer than `range`, found by a search that replays
+// the reference's opening decisions only on the ancestors of leaves within range.
+cudaError_t collide_find(const MergeBufs &m, const Tree &t, const int32_t *oparent, const int32_t *leaf_oparent,
+                         double theta, double range, cudaStream_t st, unsigned *launches);
 // Connected components of the pairs (root = smallest user index), endpoints
 // scanned into a list; counters[kMcInvolved] = its length.
 cudaError_t collide_components(const MergeBufs &m, uint32_t n, uint32_t npairs, cudaStream_t st, unsigned *launches);

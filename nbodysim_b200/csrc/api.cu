@@ -48,7 +48,6 @@ int fail(int code, const char *fmt, const char *detail = "") {
     } while (0)
 
 constexpr uint32_t kMaxParticles = 1u << 28;
-constexpr uint32_t kSpillCap = 4096;  // entries per walk warp
 constexpr unsigned kBboxBlocks = 592;
 constexpr unsigned kDiagBlocks = 296;
 constexpr uint32_t kOverlapMin = 65536;  // nbody_step_host overlaps the velocity upload from this size
@@ -71,7 +70,7 @@ struct nbody_ctx {
     uint32_t *counts = nullptr;
     TreeBuild tb{};
     double *diag_partial = nullptr;
-    int2 *spill = nullptr;
+    int2 *queue = nullptr;
     DevScalars *sc = nullptr;   // device
     DevScalars *hsc = nullptr;  // pinned mirror
     WalkLaunch wl_mixed{}, wl_fp64{};
@@ -80,7 +79,7 @@ struct nbody_ctx {
     cudaEvent_t ev[5] = {};
     nbody_stats stats{};
     unsigned long long launches = 0;  // kernels enqueued by this context
-    unsigned max_walk_warps = 0;      // spill regions allocated
+    unsigned max_walk_warps = 0;      // queues allocated
     std::vector<unsigned char> tuned_key;  // configuration the autotuner last ran for
     // adjoint state (allocated on first use)
     void *adj_arena = nullptr;
@@ -185,7 +184,7 @@ int reserve(nbody_ctx *c, uint32_t n) {
     const size_t N = cap;
     const size_t sort_blocks = (N + 4095) / 4096;
     const size_t scan_tiles = (256 * sort_blocks + 4095) / 4096 + (N + 4095) / 4096 + 8;
-    const size_t spill_entries = (size_t)c->max_walk_warps * kSpillCap;
+    const size_t queue_entries = (size_t)c->max_walk_warps * kQueueCap;
     struct Piece { void **dst; size_t bytes; };
     TreeBuild &tb = c->tb;
     Piece pieces[] = {
@@ -202,7 +201,7 @@ int reserve(nbody_ctx *c, uint32_t n) {
         {(void **)&tb.ochild, 32 * N}, {(void **)&tb.ometa, 4 * N}, {(void **)&tb.oparent, 4 * N},
         {(void **)&tb.leaf_oparent, 4 * N},
         {(void **)&tb.bbox_partial, 8 * 7 * kBboxBlocks}, {(void **)&c->diag_partial, 8 * kDiagCount * kDiagBlocks},
-        {(void **)&c->spill, 8 * spill_entries},
+        {(void **)&c->queue, 8 * queue_entries},
     };
     size_t total = 0;
     for (auto &pc : pieces) total += align256(pc.bytes);
@@ -332,7 +331,7 @@ int check_status(nbody_ctx *c) {
     if (h.status & kStatusNonFinite) return fail(NBODY_ERR_NONFINITE, "a position or mass is NaN or infinite%s");
     if (h.status & kStatusCoincident)
         return fail(NBODY_ERR_COINCIDENT, "particles coincide to 63 octree levels (the reference recurses without bound)%s");
-    if (h.status & kStatusCapacity) return fail(NBODY_ERR_CAPACITY, "walk stack spill capacity exceeded%s");
+    if (h.status & kStatusCapacity) return fail(NBODY_ERR_CAPACITY, "octree capacity exceeded%s");
     if (h.status & kStatusSortStall) return fail(NBODY_ERR_CUDA, "radix sort look-back gave up waiting%s");
     return NBODY_OK;
 }
@@ -413,9 +412,9 @@ int force_pass(nbody_ctx *c, int damping, double theta, bool fp64, bool want_vma
     a.accd = fp64 ? (acc64_out ? acc64_out : (double *)c->acc) : nullptr;
     a.counts = want_counts ? c->counts : nullptr;
     a.pot = want_pot ? c->pot : nullptr;
-    a.spill = c->spill;
-    a.spill_cap = kSpillCap;
+    a.queue = c->queue;
     a.n_groups = multi ? c->ngroups : (n + 31) / 32;
+    a.systems = multi ? c->nsys : 1;
     a.groups = multi ? c->groups : nullptr;
     a.sys_root_node = c->sys_root_node;
     a.sys_root = c->sys_root;
@@ -1011,7 +1010,7 @@ int nbody_create(const nbody_params *p, nbody_ctx **out) {
         walk_launch_shape(true, p->device, kWalkWarps, 0, &c->wl_fp64) != cudaSuccess)
         return cleanup(fail(NBODY_ERR_CUDA, "walk kernel configuration failed (%s)",
                             cudaGetErrorString(cudaGetLastError())));
-    // spill regions for the largest resident warp count any tuned shape can have
+    // walk queues for the largest resident warp count any tuned shape can have
     for (unsigned w : {1u, 2u, 4u})
         for (int fp = 0; fp < 2; fp++) {
             int mb = 0;

@@ -31,6 +31,8 @@
 // reference's opening test evaluated directly.
 #include "walk.cuh"
 
+#include <type_traits>
+
 namespace nbody {
 
 namespace {
@@ -52,13 +54,6 @@ __device__ inline float rsqrt_ftz(float x) {
 }
 
 
-// Per-warp shared memory. The stack holds nodes still to be examined with
-// the mask of lanes that reached them; the tile holds the up-to-32 internal
-// nodes being decided; the list holds accepted bodies (internal nodes a lane
-// did not open, and leaves) with the mask of lanes that take them.
-template <bool kFp64>
-struct WarpSmem;
-
 // Values that are the same for every lane of a group, kept in shared memory
 // rather than in one register per lane.
 struct GroupConsts {
@@ -66,56 +61,87 @@ struct GroupConsts {
     double S, s_theta;  // root side, root side / theta
     float box[6];       // group box of the FP32 offsets: lo x, hi x, lo y, hi y, lo z, hi z
     float pm_tol, tiny, near_r2, pad;
-    uint32_t st[6];     // per-group statistics: entries, tiles, decisions, list, near, deepest stack
+    uint32_t st[6];     // per-group statistics: entries, tiles, decisions, list, near, longest queue
 };
 
-// MIXED lists of the forward walk are stored in pairs of entries, so that the
-// packed FP32 instructions (two lanes of arithmetic each) read their operands
-// straight from two 16-byte loads: entries 2j and 2j+1 occupy 8 floats
-// (x0, x1, y0, y1, z0, z1, Gm0, Gm1) at 8j. The adjoint keeps one float4 per entry.
+// Shared memory of one warp: the tile's nodes that are decided lane by lane.
+template <bool kFp64>
+struct TileSmem;
 template <>
-struct WarpSmem<false> {
-    GroupConsts gc;
-    int2 stack[kStackCap];
+struct TileSmem<false> {
     // The tile's mixed nodes, compacted and stored in pairs: pair j holds
     // x0 x1 y0 y1 z0 z1 -q0 -q1 band0 band1 reach0 reach1 ref0 ref1 - - at 16 j
     // ((com - ref).xyz, q = (side/theta)^2, the half-width of its error band, the
     // mask of lanes that reached the node, the node). Once a pair is decided,
     // its first two words hold the two open masks.
     alignas(16) float mx[16 * 16];
-    union {
-        float4 lc[kListCap];  // adjoint: (com - ref).xyz, G m per entry
-        float lp[4 * kListCap];  // forward: entries taken by some lanes, in pairs
-    };
-    float lf[4 * kListCap];   // forward: entries taken by every lane of the group, in pairs
-    uint32_t lm[kListCap];
-    int lr[kListCap];         // node refs (adjoint mode)
-    union {
-        double4 nc[32];       // adjoint near list: com.xyz (absolute), G m
-        struct {
-            float hi[4 * kListCap];  // forward near list, in pairs: offsets rounded to FP32, G m
-            float lo[4 * kListCap];  // and what the rounding left (x, y, z; the fourth slot is 0)
-        } np;
-    };
-    uint32_t nm[kListCap];
-    int nr[32];
+};
+template <>
+struct TileSmem<true> {
+    alignas(16) double4 tc[32];  // com.xyz (absolute), side
+    int2 tr[32];                 // reach mask, node ref
 };
 
-// The paired lists and the mixed-node pairs are read with 16-byte loads.
-static_assert(offsetof(WarpSmem<false>, mx) % 16 == 0 && offsetof(WarpSmem<false>, lp) % 16 == 0 &&
-                  offsetof(WarpSmem<false>, lf) % 16 == 0 && offsetof(WarpSmem<false>, np) % 16 == 0 &&
-                  sizeof(WarpSmem<false>) % 16 == 0,
-              "16-byte shared loads need 16-byte aligned arrays");
+// Shared memory of one group: its interaction lists, rings of kCap entries that
+// are summed in batches of 32, and the sums so far. Which lists there are:
+//   MIXED forward: entries every lane takes, entries some lanes take (a lane mask
+//   each), and bodies near the group's box; MIXED adjoint: the last two; FP64: one,
+//   with masks.
+// MIXED forward lists are stored in pairs of entries, so that the packed FP32
+// instructions (two lanes of arithmetic each) read their operands straight from
+// two 16-byte loads: entries 2j and 2j+1 occupy 8 floats
+// (x0, x1, y0, y1, z0, z1, Gm0, Gm1) at 8j. The adjoint keeps one float4 per entry.
+template <bool kFp64, bool kAdj, int kCap>
+struct GroupSmem;
 
-template <>
-struct WarpSmem<true> {
+template <int kCap>
+struct GroupSmem<false, false, kCap> {
     GroupConsts gc;
-    int2 stack[kStackCap];
-    double4 tc[32];           // com.xyz (absolute), side
-    int2 tr[32];              // reach mask, node ref
-    double4 lc[kListCap];     // com.xyz (absolute), G m
-    uint32_t lm[kListCap];
-    int lr[kListCap];
+    alignas(16) float lf[4 * kCap];
+    alignas(16) float lp[4 * kCap];
+    alignas(16) float nhi[4 * kCap];  // near: offsets rounded to FP32, G m
+    alignas(16) float nlo[4 * kCap];  // and what the rounding left (x, y, z; the fourth slot is 0)
+    alignas(8) uint32_t lm[kCap];
+    alignas(8) uint32_t nm[kCap];
+    float acc[3][3][32];              // per list and component: sums of the batches so far
+};
+template <int kCap>
+struct GroupSmem<false, true, kCap> {
+    GroupConsts gc;
+    alignas(16) float4 lc[kCap];      // (com - ref).xyz, G m
+    alignas(16) double4 nc[kCap];     // near: com.xyz (absolute), G m
+    uint32_t lm[kCap], nm[kCap];
+    int lr[kCap], nr[kCap];           // node refs
+    float acc[2][3][32];
+};
+template <bool kAdj, int kCap>
+struct GroupSmem<true, kAdj, kCap> {
+    GroupConsts gc;
+    alignas(16) double4 lc[kCap];     // com.xyz (absolute), G m
+    uint32_t lm[kCap];
+    int lr[kAdj ? kCap : 1];
+    double acc[1][4][32];             // x, y, z, potential
+};
+
+// A team's block: its group, the queue, the batches summed in this round, and what
+// each warp's tile adds.
+constexpr int kTeamSlots = kTeamMaxWarps + 3;
+template <bool kFp64, bool kAdj>
+struct TeamSmem {
+    GroupSmem<kFp64, kAdj, kTeamList> g;
+    TileSmem<kFp64> tile[kTeamMaxWarps];
+    int2 queue[kQueueCap];
+    std::conditional_t<kFp64, double, float> slot[kTeamSlots][kFp64 ? 4 : 3][32];
+    alignas(16) uint32_t add[kTeamMaxWarps][4];  // entries for the three lists, children
+    uint32_t cnt[32];                 // accepted nodes per lane
+    uint32_t group;
+};
+
+// Shared memory of a warp that walks a group by itself; its queue is in global memory.
+template <bool kFp64, bool kAdj>
+struct SoloSmem {
+    GroupSmem<kFp64, kAdj, kSoloList> g;
+    TileSmem<kFp64> tile;
 };
 
 // The reference's FP64 opening test on the original doubles
@@ -146,29 +172,6 @@ __device__ inline bool ref_open(bool single, double cx, double cy, double cz, do
                                 double side, double theta, float theta_f) {
     return single ? exact_open_f32(cx, cy, cz, px, py, pz, side, theta_f)
                   : exact_open(cx, cy, cz, px, py, pz, side, theta);
-}
-
-// Moves the oldest half of a full stack to this warp's global spill region.
-template <class Sm>
-__device__ inline bool spill_out(Sm &s, int &top, uint32_t &spill_top, int2 *gspill, uint32_t spill_cap,
-                                 int lane) {
-    if (spill_top + kSpillChunk > spill_cap) return false;
-    for (int e = lane; e < kSpillChunk; e += 32) gspill[spill_top + e] = s.stack[e];
-    __syncwarp();
-    for (int e = lane; e < top - kSpillChunk; e += 32) s.stack[e] = s.stack[e + kSpillChunk];
-    __syncwarp();
-    top -= kSpillChunk;
-    spill_top += kSpillChunk;
-    return true;
-}
-
-template <class Sm>
-__device__ inline void spill_in(Sm &s, int &top, uint32_t &spill_top, const int2 *gspill, int lane) {
-    int take = min((int)spill_top, kSpillChunk);
-    for (int e = lane; e < take; e += 32) s.stack[e] = gspill[spill_top - take + e];
-    __syncwarp();
-    spill_top -= take;
-    top = take;
 }
 
 // ---- packed FP32 pairs (sm_100 f32x2: one instruction, two FP32 lanes of work)
@@ -203,12 +206,12 @@ __device__ inline void put_pair_entry(float *l, int k, float x, float y, float z
 // An offset o (FP64) as hi + lo in FP32: hi = o rounded, lo = what it left, rounded.
 __device__ inline float lo_part(double o, float hi) { return (float)(o - (double)hi); }
 
-// Gravity of the entries of a paired list on this lane's particle, two entries
-// per packed instruction. kMasked: entry k is taken iff `bit` is set in lm[k];
-// an entry not taken enters with inverse distance 0, so it adds exactly 0 even
-// when it is the lane's own leaf (distance 0). Without kMasked every entry is
-// taken. An odd count is padded with a far, massless entry. Accumulates into
-// (ax, ay, az).
+// Gravity of a batch of a paired list on this lane's particle, two entries per
+// packed instruction. kMasked: entry k is taken iff `bit` is set in lm[k]; an
+// entry not taken enters with inverse distance 0, so it adds exactly 0 even when
+// it is the lane's own leaf (distance 0). Without kMasked every entry is taken.
+// An odd count is padded with a far, massless entry. The batch's sums are returned
+// in v.
 //
 // kComp (the near list): the entry offsets are hi + lo pairs (`lo` holds the lo
 // parts in the same layout) and so is the particle's (plx, ply, plz): the
@@ -217,8 +220,8 @@ __device__ inline float lo_part(double o, float hi) { return (float)(o - (double
 // the particle gets its offset to FP32 accuracy of the offset itself.
 template <bool kDamp, bool kMasked, bool kComp = false>
 __device__ inline void force_pairs_f32(float *l, const uint32_t *lm, int count, uint32_t bit, float px, float py,
-                                       float pz, float &ax, float &ay, float &az, float *lo = nullptr,
-                                       float plx = 0.f, float ply = 0.f, float plz = 0.f) {
+                                       float pz, float (&v)[3], float *lo = nullptr, float plx = 0.f, float ply = 0.f,
+                                       float plz = 0.f) {
     if (count & 1) {
         __syncwarp();
         if ((threadIdx.x & 31) == 0) {
@@ -269,9 +272,9 @@ __device__ inline void force_pairs_f32(float *l, const uint32_t *lm, int count, 
         sz = f2fma(f, dz, sz);
     }
     float a0, a1;
-    f2unpack(sx, a0, a1); ax += a0 + a1;
-    f2unpack(sy, a0, a1); ay += a0 + a1;
-    f2unpack(sz, a0, a1); az += a0 + a1;
+    f2unpack(sx, a0, a1); v[0] = a0 + a1;
+    f2unpack(sy, a0, a1); v[1] = a0 + a1;
+    f2unpack(sz, a0, a1); v[2] = a0 + a1;
 }
 
 // Per-particle accepted-body counts of a list (only when counts are requested).
@@ -466,32 +469,95 @@ __device__ inline void force_list_f64(const double4 *lc, const uint32_t *lm, int
     }
 }
 
-template <bool kFp64, bool kDamp, bool kPot, bool kAdj, class Sm>
-__device__ inline void flush_list(Sm &s, int count, int lane, const WalkArgs &a, const double4 &b, float px, float py,
-                                  float pz, double lax, double lay, double laz, float &fax, float &fay, float &faz,
-                                  double &dax, double &day, double &daz, double &dpot, uint32_t &cnt) {
+// Sums one batch (count <= 32 entries from ring position `start`, a multiple of 32)
+// of list `list` on this lane's particle into v; cnt grows by the accepted bodies.
+template <bool kFp64, bool kDamp, bool kPot, bool kAdj, int kList, class G, typename Acc, int NC>
+__device__ inline void sum_batch(G &s, int start, int count, int lane, const WalkArgs &a, const double4 &b, float px,
+                                 float py, float pz, float plx, float ply, float plz, double lax, double lay,
+                                 double laz, Acc (&v)[NC], uint32_t &cnt) {
     const uint32_t bit = 1u << lane;
-    if constexpr (kAdj) {
-        if constexpr (kFp64)
-            adj_list_f64<kDamp>(s.lc, s.lm, s.lr, count, lane, b.x, b.y, b.z, lax, lay, laz, dax, day, daz, a.adj_node,
-                                a.adj_leaf);
-        else
-            adj_list_f32<kDamp>(s.lc, s.lm, s.lr, count, lane, px, py, pz, (float)lax, (float)lay, (float)laz, fax, fay,
-                                faz, a.adj_node, a.adj_leaf);
+#pragma unroll
+    for (int c = 0; c < NC; c++) v[c] = Acc(0);
+    if constexpr (kFp64) {
+        if constexpr (kAdj) {
+            adj_list_f64<kDamp>(s.lc + start, s.lm + start, s.lr + start, count, lane, b.x, b.y, b.z, lax, lay, laz,
+                                v[0], v[1], v[2], a.adj_node, a.adj_leaf);
+        } else {
+            double pot = 0.0;
+            force_list_f64<kDamp, kPot>(s.lc + start, s.lm + start, count, lane, b.x, b.y, b.z, v[0], v[1], v[2], pot);
+            if constexpr (NC > 3) v[3] = pot;
+        }
+        if (a.counts) cnt += count_list(s.lm + start, count, bit);
+    } else if constexpr (kAdj) {
+        if constexpr (kList == 0) {
+            adj_list_f32<kDamp>(s.lc + start, s.lm + start, s.lr + start, count, lane, px, py, pz, (float)lax,
+                                (float)lay, (float)laz, v[0], v[1], v[2], a.adj_node, a.adj_leaf);
+            if (a.counts) cnt += count_list(s.lm + start, count, bit);
+        } else {
+            adj_near_f32<kDamp>(s.nc + start, s.nm + start, s.nr + start, count, lane, b.x, b.y, b.z, (float)lax,
+                                (float)lay, (float)laz, v[0], v[1], v[2], a.adj_node, a.adj_leaf);
+            if (a.counts) cnt += count_list(s.nm + start, count, bit);
+        }
     } else {
-        if constexpr (kFp64) force_list_f64<kDamp, kPot>(s.lc, s.lm, count, lane, b.x, b.y, b.z, dax, day, daz, dpot);
-        else force_pairs_f32<kDamp, true>(s.lp, s.lm, count, bit, px, py, pz, fax, fay, faz);
+        if constexpr (kList == 0) {
+            force_pairs_f32<kDamp, false>(s.lf + 4 * start, nullptr, count, 0u, px, py, pz, v);
+            cnt += count;
+        } else if constexpr (kList == 1) {
+            force_pairs_f32<kDamp, true>(s.lp + 4 * start, s.lm + start, count, bit, px, py, pz, v);
+            if (a.counts) cnt += count_list(s.lm + start, count, bit);
+        } else {
+            force_pairs_f32<kDamp, true, true>(s.nhi + 4 * start, s.nm + start, count, bit, px, py, pz, v,
+                                               s.nlo + 4 * start, plx, ply, plz);
+            if (a.counts) cnt += count_list(s.nm + start, count, bit);
+        }
     }
-    if (a.counts) cnt += count_list(s.lm, count, bit);
 }
 
-template <bool kFp64, bool kDamp, bool kPot, bool kAdj, bool kStats>
-__global__ void __launch_bounds__(kWalkMaxWarps * 32) k_walk(WalkArgs a) {
+// The walk of one group of up to 32 particles, by one warp (kTeam false) or by the
+// warps of a block together (kTeam true).
+//
+// Both do the same arithmetic in the same order. The entries still to be examined
+// wait in a queue, first in first out, so the sequence in which they are examined,
+// and with it the sequence of every interaction list, does not depend on how many
+// are examined at a time; each list is summed in batches of 32 consecutive entries,
+// the batches' sums are added in order, and the lists' sums last. (Past kQueueWide
+// waiting entries the newest go first, one tile at a time, which bounds the queue;
+// a team takes no more tiles at once than keep the order of one warp's walk.)
+//
+// Bound of few groups: the serial chain of one group's tiles (~3 us each at one warp
+// per scheduler; 11% of issue slots used on a shell of 20,011), which a team of four
+// cuts to a third; of many: instruction issue (67% of slots), where one warp each
+// needs no barriers. Teams of 2, 6 and 8 warps were slower (5000 particles: 79, 51,
+// 55 us against 51 with four; 65,536: 291, 330, 446 against 258). A stack cut into
+// parts for several warps, last in first out, was as fast for few groups, but one
+// warp that has to repeat its order of sums for an ensemble took 12 to 30% longer.
+template <bool kFp64, bool kDamp, bool kPot, bool kAdj, bool kStats, bool kTeam>
+__global__ void __launch_bounds__((kTeam ? kTeamMaxWarps : kWalkMaxWarps) * 32) k_walk(WalkArgs a) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     griddep();
-    using Sm = WarpSmem<kFp64>;
+    using Acc = std::conditional_t<kFp64, double, float>;
+    using Team = TeamSmem<kFp64, kAdj>;
+    using Solo = SoloSmem<kFp64, kAdj>;
+    constexpr int kLists = kFp64 ? 1 : kAdj ? 2 : 3;
+    constexpr int NC = kPot ? 4 : 3;
+    constexpr uint32_t kCap = kTeam ? kTeamList : kSoloList;
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    Sm &s = reinterpret_cast<Sm *>(smem_raw)[wid];
+    Team &tm = *reinterpret_cast<Team *>(smem_raw);
+    Solo &solo = reinterpret_cast<Solo *>(smem_raw)[kTeam ? 0 : wid];
+    auto &s = [&]() -> auto & {
+        if constexpr (kTeam) return tm.g;
+        else return solo.g;
+    }();
+    auto &tile = [&]() -> auto & {
+        if constexpr (kTeam) return tm.tile[wid];
+        else return solo.tile;
+    }();
+    int2 *const queue = kTeam ? tm.queue : a.queue + (size_t)(blockIdx.x * (blockDim.x >> 5) + wid) * kQueueCap;
+    const uint32_t w = kTeam ? wid : 0, W = kTeam ? blockDim.x >> 5 : 1;  // this warp within the team
+    auto sync = [] {
+        if constexpr (kTeam) __syncthreads();
+        else __syncwarp();
+    };
     const Tree &t = a.t;
     const uint32_t n = t.n;
     const bool single = a.single != 0;
@@ -501,14 +567,20 @@ __global__ void __launch_bounds__(kWalkMaxWarps * 32) k_walk(WalkArgs a) {
     // the FLOAT build's (~6.3 float ulps of (side/theta)^2)
     const double grp_rel = single ? 1e-6 : 1e-12;
     const double S1 = t.sc->root_side;
-    int2 *gspill = a.spill + (size_t)(blockIdx.x * (blockDim.x >> 5) + wid) * a.spill_cap;
     const unsigned FULL = 0xffffffffu;
     const uint32_t lt = (1u << lane) - 1u;
 
     for (;;) {
         uint32_t g = 0;
-        if (lane == 0) g = atomicAdd(&t.sc->group_counter, 1u);
-        g = __shfl_sync(FULL, g, 0);
+        if constexpr (kTeam) {
+            __syncthreads();  // the last group's shared memory is no longer read
+            if (threadIdx.x == 0) tm.group = atomicAdd(&t.sc->group_counter, 1u);
+            __syncthreads();
+            g = tm.group;
+        } else {
+            if (lane == 0) g = atomicAdd(&t.sc->group_counter, 1u);
+            g = __shfl_sync(FULL, g, 0);
+        }
         if (g >= a.n_groups) break;
 
         uint32_t g0, gcount;
@@ -571,42 +643,65 @@ __global__ void __launch_bounds__(kWalkMaxWarps * 32) k_walk(WalkArgs a) {
             loz = warp_minf(pz); hiz = warp_maxf(pz);
         }
 
-        if (lane == 0) {
-            s.gc.ref[0] = rx; s.gc.ref[1] = ry; s.gc.ref[2] = rz;
-            s.gc.S = S; s.gc.s_theta = s_theta;
-            s.gc.box[0] = lox; s.gc.box[1] = hix; s.gc.box[2] = loy;
-            s.gc.box[3] = hiy; s.gc.box[4] = loz; s.gc.box[5] = hiz;
-            s.gc.pm_tol = pm_tol; s.gc.tiny = tiny; s.gc.near_r2 = near_r2;
-            if constexpr (kStats)
-                for (int q = 0; q < 6; q++) s.gc.st[q] = 0u;
+        if (w == 0) {
+            if (lane == 0) {
+                s.gc.ref[0] = rx; s.gc.ref[1] = ry; s.gc.ref[2] = rz;
+                s.gc.S = S; s.gc.s_theta = s_theta;
+                s.gc.box[0] = lox; s.gc.box[1] = hix; s.gc.box[2] = loy;
+                s.gc.box[3] = hiy; s.gc.box[4] = loz; s.gc.box[5] = hiz;
+                s.gc.pm_tol = pm_tol; s.gc.tiny = tiny; s.gc.near_r2 = near_r2;
+                if constexpr (kStats)
+                    for (int q = 0; q < 6; q++) s.gc.st[q] = 0u;
+                queue[0] = make_int2(root, (int)vmask);
+            }
+#pragma unroll
+            for (int l = 0; l < kLists; l++)
+#pragma unroll
+                for (int c = 0; c < NC; c++) s.acc[l][c][lane] = Acc(0);
+            if constexpr (kTeam) tm.cnt[lane] = 0u;
         }
-        float fax = 0.f, fay = 0.f, faz = 0.f;
-        double dax = 0.0, day = 0.0, daz = 0.0, dpot = 0.0;
         uint32_t cnt = 0, nint = 0, nfallback = 0;
-        int top = 0, list_top = 0, full_top = 0, near_top = 0;
-        uint32_t spill_top = 0;
-        bool failed = false;
-        if (root >= 0) {
-            if (lane == 0) s.stack[0] = make_int2(root, (int)vmask);
-            top = 1;
-        }
-        __syncwarp();
+        uint32_t head = 0, qn = root >= 0 ? 1u : 0u;       // the queue: first entry, entries
+        uint32_t lstart[3] = {0, 0, 0}, lcount[3] = {0, 0, 0};  // each list's ring: first entry, entries
+        // the next tile's entries, loaded a tile early where the queue (in global memory)
+        // holds them all already: -1 to -2% walk time
+        int2 ahead = make_int2(0, 0);
+        bool have_ahead = false;
+        sync();
 
-        while (top > 0 || spill_top > 0) {
-            if (top == 0) spill_in(s, top, spill_top, gspill, lane);
-            const int cntt = min(top, 32);
-            const int base = top - cntt;
-            top = base;
-            if (kStats && lane == 0) { s.gc.st[0] += cntt; s.gc.st[1] += 1u; }
+        while (qn > 0) {
+            uint32_t base, take;
+            if (qn <= kQueueWide) {
+                // a team takes whole tiles, as many as cannot take the queue past kQueueWide
+                // between them (one warp would turn to the newest entries there)
+                const uint32_t tiles = kTeam ? max(1u, min(min(W, qn / 32u), 1u + (kQueueWide - qn) / 224u)) : 1u;
+                base = head;
+                take = min(qn, 32u * tiles);
+                head += take;
+            } else {
+                // the newest entries; fewer as the queue fills, down to a depth-first
+                // descent of one at a time, for which kQueueReserve is room
+                const int room = ((int)(kQueueCap - kQueueReserve) - (int)qn) / 8;
+                take = (uint32_t)max(1, min(32, room));
+                base = head + qn - take;
+            }
+            qn -= take;
+            const int cntt = take > 32u * w ? (int)min(32u, take - 32u * w) : 0;
+            if (kStats && lane == 0 && cntt > 0) {
+                atomicAdd(&s.gc.st[0], (uint32_t)cntt);
+                atomicAdd(&s.gc.st[1], 1u);
+            }
 
-            // ---- stage: lane k takes stack entry k
+            // ---- stage: lane k takes the tile's entry k
             bool is_int = false;
             int4 ch0 = make_int4(0, 0, 0, 0), ch1 = make_int4(0, 0, 0, 0);
             uint32_t reach = 0;
             int nch = 0, ref = 0;
             double cx = 0, cy = 0, cz = 0, m = 0, so = 0;
             if (lane < cntt) {
-                const int2 e = s.stack[base + lane];
+                const int2 e = !kTeam && have_ahead && base == head - 32u
+                                   ? ahead
+                                   : queue[(base + 32u * w + lane) & (kQueueCap - 1)];
                 ref = e.x;
                 reach = (uint32_t)e.y;
                 if (ref >= 0) {
@@ -625,6 +720,10 @@ __global__ void __launch_bounds__(kWalkMaxWarps * 32) k_walk(WalkArgs a) {
                     const uint32_t own = (uint32_t)(~ref) - g0;  // a leaf of this group: not its own lane
                     if (own < 32u) reach &= ~(1u << own);
                 }
+            }
+            if constexpr (!kTeam) {
+                have_ahead = qn >= 32u;
+                if (have_ahead) ahead = queue[(head + lane) & (kQueueCap - 1)];
             }
             float fcx = 0.f, fcy = 0.f, fcz = 0.f;
             if constexpr (!kFp64) {
@@ -676,11 +775,11 @@ __global__ void __launch_bounds__(kWalkMaxWarps * 32) k_walk(WalkArgs a) {
 
             // ---- decide the mixed nodes of the tile, lane by lane
             const uint32_t intm = __ballot_sync(FULL, mixed);
-            if (kStats && lane == 0) s.gc.st[2] += __popc(intm);
+            if (kStats && lane == 0) atomicAdd(&s.gc.st[2], (uint32_t)__popc(intm));
             if (intm) {
                 if constexpr (kFp64) {
-                    s.tc[lane] = make_double4(cx, cy, cz, s.gc.S * so);
-                    s.tr[lane] = make_int2((int)reach, ref);
+                    tile.tc[lane] = make_double4(cx, cy, cz, s.gc.S * so);
+                    tile.tr[lane] = make_int2((int)reach, ref);
                     __syncwarp();
                 }
                 if constexpr (kFp64) {
@@ -689,8 +788,8 @@ __global__ void __launch_bounds__(kWalkMaxWarps * 32) k_walk(WalkArgs a) {
                     while (mm) {
                         const int k = __ffs(mm) - 1;
                         mm &= mm - 1;
-                        const double4 c = s.tc[k];
-                        const uint32_t rk = (uint32_t)s.tr[k].x;
+                        const double4 c = tile.tc[k];
+                        const uint32_t rk = (uint32_t)tile.tr[k].x;
                         const bool open = ref_open(single, c.x, c.y, c.z, b.x, b.y, b.z, c.w, theta, theta_f);
                         const uint32_t om = __ballot_sync(FULL, open) & rk;
                         if (lane == k) my_open = om;
@@ -704,13 +803,13 @@ __global__ void __launch_bounds__(kWalkMaxWarps * 32) k_walk(WalkArgs a) {
                     const int nmix = __popc(intm);
                     const int mpos = __popc(intm & lt);
                     if (mixed) {
-                        float *e = s.mx + 16 * (mpos >> 1) + (mpos & 1);
+                        float *e = tile.mx + 16 * (mpos >> 1) + (mpos & 1);
                         e[0] = fcx; e[2] = fcy; e[4] = fcz; e[6] = -qf;
                         e[8] = band; e[10] = __uint_as_float(reach); e[12] = __int_as_float(ref);
                     }
                     if (lane == 0 && (nmix & 1)) {
                         // pad an odd count with an entry no lane reached
-                        float *e = s.mx + 16 * (nmix >> 1) + 1;
+                        float *e = tile.mx + 16 * (nmix >> 1) + 1;
                         e[0] = 0.f; e[2] = 0.f; e[4] = 0.f; e[6] = 0.f;
                         e[8] = 0.f; e[10] = 0.f; e[12] = 0.f;
                     }
@@ -719,7 +818,7 @@ __global__ void __launch_bounds__(kWalkMaxWarps * 32) k_walk(WalkArgs a) {
                     const uint64_t npx = f2pack(-px, -px), npy = f2pack(-py, -py), npz = f2pack(-pz, -pz);
                     const uint32_t bit = 1u << lane;
                     for (int k = 0; k < nmix; k += 2) {
-                        float *pr = s.mx + 8 * k;
+                        float *pr = tile.mx + 8 * k;
                         const float4 A = *reinterpret_cast<const float4 *>(pr);      // x0 x1 y0 y1
                         const float4 B = *reinterpret_cast<const float4 *>(pr + 4);  // z0 z1 -q0 -q1
                         const float4 C = *reinterpret_cast<const float4 *>(pr + 8);  // band0 band1 reach0 reach1
@@ -758,15 +857,16 @@ __global__ void __launch_bounds__(kWalkMaxWarps * 32) k_walk(WalkArgs a) {
                         if (lane == 0) *reinterpret_cast<uint2 *>(pr) = make_uint2(om1, om2);
                     }
                     __syncwarp();
-                    if (mixed) my_open = __float_as_uint(s.mx[16 * (mpos >> 1) + (mpos & 1)]);
+                    if (mixed) my_open = __float_as_uint(tile.mx[16 * (mpos >> 1) + (mpos & 1)]);
                 }
                 __syncwarp();
             }
 
-            // ---- accepted bodies -> interaction list (compacted across lanes).
+            // ---- accepted bodies -> interaction lists (compacted across lanes).
             // MIXED: a body closer to the group's box than 2^-9 of the group's
             // extent would lose too many bits in FP32 offsets (and could give a
-            // zero r^2); it goes to the near list, whose offsets are taken in FP64.
+            // zero r^2); it goes to the near list, whose offsets keep FP32 accuracy
+            // of the offset itself.
             const uint32_t accm = reach & ~my_open;
             nint += __popc(accm);
             bool near = false;
@@ -781,142 +881,190 @@ __global__ void __launch_bounds__(kWalkMaxWarps * 32) k_walk(WalkArgs a) {
                     near = r2box < s.gc.near_r2;
                 }
             }
-            if constexpr (!kFp64 && !kAdj) {
-                // entries every lane of the group takes go to a list without masks
-                const bool take = accm != 0 && !near;
-                const bool all = take && accm == vmask;
-                const uint32_t fmk = __ballot_sync(FULL, all);
-                const uint32_t pmk = __ballot_sync(FULL, take && !all);
-                const float gmf = (float)(kG * m);
-                if (all) {
-                    put_pair_entry(s.lf, full_top + __popc(fmk & lt), fcx, fcy, fcz, gmf);
-                } else if (take) {
-                    const int pos = list_top + __popc(pmk & lt);
-                    put_pair_entry(s.lp, pos, fcx, fcy, fcz, gmf);
-                    s.lm[pos] = accm;
-                }
-                full_top += __popc(fmk);
-                list_top += __popc(pmk);
-                if (kStats && lane == 0) s.gc.st[3] += __popc(fmk) + __popc(pmk);
-            } else {
-                const uint32_t am = __ballot_sync(FULL, accm != 0 && !near);
-                if (accm && !near) {
-                    const int pos = list_top + __popc(am & lt);
-                    if constexpr (kFp64) s.lc[pos] = make_double4(cx, cy, cz, kG * m);
-                    else s.lc[pos] = make_float4(fcx, fcy, fcz, (float)(kG * m));
-                    s.lm[pos] = accm;
-                    if constexpr (kAdj) s.lr[pos] = ref;
-                }
-                list_top += __popc(am);
-                if (kStats && lane == 0) s.gc.st[3] += __popc(am);
-            }
-            if constexpr (!kFp64 && !kAdj) {
-                // forward: near bodies collect in their own paired list, offsets as hi + lo
-                const uint32_t nmk = __ballot_sync(FULL, near);
-                if (nmk) {
-                    if (near) {
-                        const int pos = near_top + __popc(nmk & lt);
-                        const double ox = cx - s.gc.ref[0], oy = cy - s.gc.ref[1], oz = cz - s.gc.ref[2];
-                        put_pair_entry(s.np.hi, pos, fcx, fcy, fcz, (float)(kG * m));
-                        put_pair_entry(s.np.lo, pos, lo_part(ox, fcx), lo_part(oy, fcy), lo_part(oz, fcz), 0.f);
-                        s.nm[pos] = accm;
-                    }
-                    near_top += __popc(nmk);
-                    if (kStats && lane == 0) s.gc.st[4] += __popc(nmk);
-                }
-            } else if constexpr (!kFp64) {
-                const uint32_t nmk = __ballot_sync(FULL, near);
-                if (nmk) {
-                    if (near) {
-                        const int pos = __popc(nmk & lt);
-                        s.nc[pos] = make_double4(cx, cy, cz, kG * m);
-                        s.nm[pos] = accm;
-                        s.nr[pos] = ref;
-                    }
-                    __syncwarp();
-                    adj_near_f32<kDamp>(s.nc, s.nm, s.nr, __popc(nmk), lane, b.x, b.y, b.z, (float)lax, (float)lay,
-                                        (float)laz, fax, fay, faz, a.adj_node, a.adj_leaf);
-                    if (a.counts) cnt += count_list(s.nm, __popc(nmk), 1u << lane);
-                    if (kStats && lane == 0) s.gc.st[4] += __popc(nmk);
-                    __syncwarp();
-                }
-            }
-
-            // ---- children of opened nodes -> stack
+            // entries every lane of the group takes go to a list without masks (MIXED forward)
+            const bool take_it = accm != 0 && !near;
+            const bool all = !kFp64 && !kAdj && take_it && accm == vmask;
+            const uint32_t amk = !kFp64 && !kAdj ? __ballot_sync(FULL, all) : 0u;
+            const uint32_t pmk = __ballot_sync(FULL, take_it && !all);
+            const uint32_t nmk = !kFp64 ? __ballot_sync(FULL, near) : 0u;
             // exclusive prefix of the child counts (0..8) from four independent ballots of their bits
             const int myn = my_open ? nch : 0;
             const uint32_t q0 = __ballot_sync(FULL, myn & 1), q1 = __ballot_sync(FULL, myn & 2),
                            q2 = __ballot_sync(FULL, myn & 4), q3 = __ballot_sync(FULL, myn & 8);
-            const int pre = __popc(q0 & lt) + 2 * __popc(q1 & lt) + 4 * __popc(q2 & lt) + 8 * __popc(q3 & lt);
-            const int total = __popc(q0) + 2 * __popc(q1) + 4 * __popc(q2) + 8 * __popc(q3);
-            if (total > 0) {
-                if (top + total > kStackCap) {
-                    if (!spill_out(s, top, spill_top, gspill, a.spill_cap, lane)) {
-                        failed = true;
-                        break;
+            const uint32_t pre = __popc(q0 & lt) + 2 * __popc(q1 & lt) + 4 * __popc(q2 & lt) + 8 * __popc(q3 & lt);
+            uint32_t add_a = __popc(amk), add_p = __popc(pmk), add_n = __popc(nmk);
+            uint32_t add_c = __popc(q0) + 2 * __popc(q1) + 4 * __popc(q2) + 8 * __popc(q3);
+            if (kStats && lane == 0) {
+                atomicAdd(&s.gc.st[3], add_a + add_p);
+                atomicAdd(&s.gc.st[4], add_n);
+            }
+            // a team's warps append in the order of their tiles
+            uint32_t off_a = 0, off_p = 0, off_n = 0, off_c = 0;
+            if constexpr (kTeam) {
+                if (lane == 0) *reinterpret_cast<uint4 *>(tm.add[w]) = make_uint4(add_a, add_p, add_n, add_c);
+                __syncthreads();
+                add_a = add_p = add_n = add_c = 0;
+                for (uint32_t q = 0; q < W; q++) {
+                    const uint4 u = *reinterpret_cast<const uint4 *>(tm.add[q]);
+                    if (q == w) { off_a = add_a; off_p = add_p; off_n = add_n; off_c = add_c; }
+                    add_a += u.x; add_p += u.y; add_n += u.z; add_c += u.w;
+                }
+            }
+            auto slot_of = [&](int l, uint32_t off, uint32_t mk) -> int {
+                const uint32_t q = lstart[l] + lcount[l] + off + __popc(mk & lt);
+                return (int)(q >= kCap ? q - kCap : q);
+            };
+            if constexpr (kFp64) {
+                if (take_it) {
+                    const int pos = slot_of(0, off_p, pmk);
+                    s.lc[pos] = make_double4(cx, cy, cz, kG * m);
+                    s.lm[pos] = accm;
+                    if constexpr (kAdj) s.lr[pos] = ref;
+                }
+                lcount[0] += add_p;
+            } else if constexpr (kAdj) {
+                if (take_it) {
+                    const int pos = slot_of(0, off_p, pmk);
+                    s.lc[pos] = make_float4(fcx, fcy, fcz, (float)(kG * m));
+                    s.lm[pos] = accm;
+                    s.lr[pos] = ref;
+                } else if (near) {
+                    const int pos = slot_of(1, off_n, nmk);
+                    s.nc[pos] = make_double4(cx, cy, cz, kG * m);
+                    s.nm[pos] = accm;
+                    s.nr[pos] = ref;
+                }
+                lcount[0] += add_p;
+                lcount[1] += add_n;
+            } else {
+                const float gmf = (float)(kG * m);
+                if (all) {
+                    put_pair_entry(s.lf, slot_of(0, off_a, amk), fcx, fcy, fcz, gmf);
+                } else if (take_it) {
+                    const int pos = slot_of(1, off_p, pmk);
+                    put_pair_entry(s.lp, pos, fcx, fcy, fcz, gmf);
+                    s.lm[pos] = accm;
+                }
+                if (nmk && near) {
+                    const int pos = slot_of(2, off_n, nmk);
+                    const double ox = cx - s.gc.ref[0], oy = cy - s.gc.ref[1], oz = cz - s.gc.ref[2];
+                    put_pair_entry(s.nhi, pos, fcx, fcy, fcz, gmf);
+                    put_pair_entry(s.nlo, pos, lo_part(ox, fcx), lo_part(oy, fcy), lo_part(oz, fcz), 0.f);
+                    s.nm[pos] = accm;
+                }
+                lcount[0] += add_a;
+                lcount[1] += add_p;
+                lcount[2] += add_n;
+            }
+
+            // ---- children of opened nodes -> queue
+            if (myn > 0) {
+                const uint32_t at = head + qn + off_c + pre;
+                const int om = (int)my_open;
+                queue[at & (kQueueCap - 1)] = make_int2(ch0.x, om);
+                if (myn > 1) queue[(at + 1) & (kQueueCap - 1)] = make_int2(ch0.y, om);
+                if (myn > 2) queue[(at + 2) & (kQueueCap - 1)] = make_int2(ch0.z, om);
+                if (myn > 3) queue[(at + 3) & (kQueueCap - 1)] = make_int2(ch0.w, om);
+                if (myn > 4) queue[(at + 4) & (kQueueCap - 1)] = make_int2(ch1.x, om);
+                if (myn > 5) queue[(at + 5) & (kQueueCap - 1)] = make_int2(ch1.y, om);
+                if (myn > 6) queue[(at + 6) & (kQueueCap - 1)] = make_int2(ch1.z, om);
+                if (myn > 7) queue[(at + 7) & (kQueueCap - 1)] = make_int2(ch1.w, om);
+            }
+            qn += add_c;
+            if (kStats && lane == 0) atomicMax(&s.gc.st[5], qn);
+            sync();
+
+            // ---- the lists' full batches
+            if constexpr (!kTeam) {
+                Acc v[NC];
+                auto solo_batch = [&](auto L) {
+                    constexpr int l = decltype(L)::value;
+                    if (lcount[l] < 32u) return;
+                    sum_batch<kFp64, kDamp, kPot, kAdj, l>(s, (int)lstart[l], 32, lane, a, b, px, py, pz, plx, ply, plz,
+                                                           lax, lay, laz, v, cnt);
+#pragma unroll
+                    for (int c = 0; c < NC; c++) s.acc[l][c][lane] += v[c];
+                    lstart[l] = lstart[l] + 32u >= kCap ? lstart[l] + 32u - kCap : lstart[l] + 32u;
+                    lcount[l] -= 32u;
+                    __syncwarp();
+                };
+                solo_batch(std::integral_constant<int, 0>{});
+                if constexpr (kLists > 1) solo_batch(std::integral_constant<int, 1>{});
+                if constexpr (kLists > 2) solo_batch(std::integral_constant<int, 2>{});
+            } else {
+                uint32_t nb = 0;
+#pragma unroll
+                for (int l = 0; l < kLists; l++) nb += lcount[l] >> 5;
+                if (nb > 0) {
+                    // batch q of the round (list by list) goes to warp q mod W
+                    uint32_t q0_ = 0;
+                    auto team_batches = [&](auto L) {
+                        constexpr int l = decltype(L)::value;
+                        const uint32_t k = lcount[l] >> 5;
+                        for (uint32_t i = (w + W - q0_ % W) % W; i < k; i += W) {
+                            const uint32_t q = lstart[l] + 32u * i;
+                            Acc v[NC];
+                            sum_batch<kFp64, kDamp, kPot, kAdj, l>(s, (int)(q >= kCap ? q - kCap : q), 32, lane, a, b, px,
+                                                                   py, pz, plx, ply, plz, lax, lay, laz, v, cnt);
+#pragma unroll
+                            for (int c = 0; c < NC; c++) tm.slot[q0_ + i][c][lane] = v[c];
+                        }
+                        q0_ += k;
+                    };
+                    team_batches(std::integral_constant<int, 0>{});
+                    if constexpr (kLists > 1) team_batches(std::integral_constant<int, 1>{});
+                    if constexpr (kLists > 2) team_batches(std::integral_constant<int, 2>{});
+                    __syncthreads();
+                    q0_ = 0;
+#pragma unroll
+                    for (int l = 0; l < kLists; l++) {
+                        const uint32_t k = lcount[l] >> 5;
+                        if ((uint32_t)l % W == w) {
+                            for (uint32_t i = 0; i < k; i++)
+#pragma unroll
+                                for (int c = 0; c < NC; c++) s.acc[l][c][lane] += tm.slot[q0_ + i][c][lane];
+                        }
+                        q0_ += k;
+                        lstart[l] += 32u * k;
+                        if (lstart[l] >= kCap) lstart[l] -= kCap;
+                        lcount[l] &= 31u;
                     }
                 }
-                int2 *dst = s.stack + top + pre;
-                const int om = (int)my_open;
-                if (myn > 0) dst[0] = make_int2(ch0.x, om);
-                if (myn > 1) dst[1] = make_int2(ch0.y, om);
-                if (myn > 2) dst[2] = make_int2(ch0.z, om);
-                if (myn > 3) dst[3] = make_int2(ch0.w, om);
-                if (myn > 4) dst[4] = make_int2(ch1.x, om);
-                if (myn > 5) dst[5] = make_int2(ch1.y, om);
-                if (myn > 6) dst[6] = make_int2(ch1.z, om);
-                if (myn > 7) dst[7] = make_int2(ch1.w, om);
-                top += total;
-                if (kStats && lane == 0) s.gc.st[5] = max(s.gc.st[5], (uint32_t)(top + (int)spill_top));
             }
-            __syncwarp();
+        }
 
-            // ---- forces once a list is long enough
-            if (list_top >= kListFlush) {
-                flush_list<kFp64, kDamp, kPot, kAdj>(s, list_top, lane, a, b, px, py, pz, lax, lay, laz, fax, fay, faz,
-                                                      dax, day, daz, dpot, cnt);
-                list_top = 0;
-                __syncwarp();
-            }
-            if constexpr (!kFp64 && !kAdj) {
-                if (full_top >= kListFlush) {
-                    force_pairs_f32<kDamp, false>(s.lf, nullptr, full_top, 0u, px, py, pz, fax, fay, faz);
-                    cnt += full_top;
-                    full_top = 0;
-                    __syncwarp();
-                }
-                if (near_top >= kListFlush) {
-                    force_pairs_f32<kDamp, true, true>(s.np.hi, s.nm, near_top, 1u << lane, px, py, pz, fax, fay, faz,
-                                                       s.np.lo, plx, ply, plz);
-                    if (a.counts) cnt += count_list(s.nm, near_top, 1u << lane);
-                    near_top = 0;
-                    __syncwarp();
-                }
-            }
+        // ---- what is left in the lists
+        {
+            Acc v[NC];
+            auto rest = [&](auto L) {
+                constexpr int l = decltype(L)::value;
+                if (lcount[l] == 0u || (kTeam && (uint32_t)l % W != w)) return;
+                sum_batch<kFp64, kDamp, kPot, kAdj, l>(s, (int)lstart[l], (int)lcount[l], lane, a, b, px, py, pz, plx, ply,
+                                                       plz, lax, lay, laz, v, cnt);
+#pragma unroll
+                for (int c = 0; c < NC; c++) s.acc[l][c][lane] += v[c];
+            };
+            rest(std::integral_constant<int, 0>{});
+            if constexpr (kLists > 1) rest(std::integral_constant<int, 1>{});
+            if constexpr (kLists > 2) rest(std::integral_constant<int, 2>{});
         }
-        if (failed && lane == 0) atomicOr(&t.sc->status, kStatusCapacity);
-        if (list_top > 0) {
-            flush_list<kFp64, kDamp, kPot, kAdj>(s, list_top, lane, a, b, px, py, pz, lax, lay, laz, fax, fay, faz,
-                                                  dax, day, daz, dpot, cnt);
+        if constexpr (kTeam) {
+            if (a.counts) atomicAdd(&tm.cnt[lane], cnt);
+            __syncthreads();
+            cnt = tm.cnt[lane];
         }
-        if constexpr (!kFp64 && !kAdj) {
-            if (full_top > 0) {
-                force_pairs_f32<kDamp, false>(s.lf, nullptr, full_top, 0u, px, py, pz, fax, fay, faz);
-                cnt += full_top;
-            }
-            if (near_top > 0) {
-                force_pairs_f32<kDamp, true, true>(s.np.hi, s.nm, near_top, 1u << lane, px, py, pz, fax, fay, faz,
-                                                   s.np.lo, plx, ply, plz);
-                if (a.counts) cnt += count_list(s.nm, near_top, 1u << lane);
-            }
-        }
-        __syncwarp();
 
         // ---- epilogue: results in the caller's particle order
-        double ax, ay, az;
-        if constexpr (kFp64) { ax = dax; ay = day; az = daz; }
-        else { ax = fax; ay = fay; az = faz; }
-        if (valid) {
+        double ax = 0.0, ay = 0.0, az = 0.0;
+#pragma unroll
+        for (int l = 0; l < kLists; l++) {
+            ax += (double)s.acc[l][0][lane];
+            ay += (double)s.acc[l][1][lane];
+            az += (double)s.acc[l][2][lane];
+        }
+        const float fax = (float)ax, fay = (float)ay, faz = (float)az;
+        if constexpr (!kFp64) { ax = fax; ay = fay; az = faz; }
+        if (valid && w == 0) {
             const uint32_t ui = t.sidx[j];
             if constexpr (kAdj) {
                 if constexpr (kFp64) {
@@ -931,7 +1079,7 @@ __global__ void __launch_bounds__(kWalkMaxWarps * 32) k_walk(WalkArgs a) {
             }
             if (a.counts) a.counts[ui] = cnt;
             if constexpr (kPot) {
-                if (a.pot) a.pot[ui] = -dpot;
+                if (a.pot) a.pot[ui] = -s.acc[0][3][lane];
             }
         }
         unsigned long long wc = nint;
@@ -944,71 +1092,106 @@ __global__ void __launch_bounds__(kWalkMaxWarps * 32) k_walk(WalkArgs a) {
             atomicAdd(&t.sc->interactions, wc);
             atomicAdd(&t.sc->interactions_total, wc);
             if (wf) atomicAdd(&t.sc->fallback_tests, wf);
-            if constexpr (kStats) {
-                atomicAdd(&t.sc->walk_entries, (unsigned long long)s.gc.st[0]);
-                atomicAdd(&t.sc->walk_tiles, (unsigned long long)s.gc.st[1]);
-                atomicAdd(&t.sc->walk_decisions, (unsigned long long)s.gc.st[2]);
-                atomicAdd(&t.sc->walk_list, (unsigned long long)s.gc.st[3]);
-                if (s.gc.st[4]) atomicAdd(&t.sc->walk_near, (unsigned long long)s.gc.st[4]);
-                atomicMax(&t.sc->max_stack, s.gc.st[5]);
+            if (w == 0) {
+                if constexpr (kStats) {
+                    atomicAdd(&t.sc->walk_entries, (unsigned long long)s.gc.st[0]);
+                    atomicAdd(&t.sc->walk_tiles, (unsigned long long)s.gc.st[1]);
+                    atomicAdd(&t.sc->walk_decisions, (unsigned long long)s.gc.st[2]);
+                    atomicAdd(&t.sc->walk_list, (unsigned long long)s.gc.st[3]);
+                    if (s.gc.st[4]) atomicAdd(&t.sc->walk_near, (unsigned long long)s.gc.st[4]);
+                    atomicMax(&t.sc->max_stack, s.gc.st[5]);
+                }
+                if (!kAdj && a.track_max_acc) atomic_max_nonneg(&t.sc->max_acc_bits, amag);
             }
-            if (!kAdj && a.track_max_acc) atomic_max_nonneg(&t.sc->max_acc_bits, amag);
         }
+        if constexpr (!kTeam) __syncwarp();
     }
 }
 
 // Potentials (diagnostics) are summed by the FP64 form only. The walk's
-// statistics (entries, tiles, decisions, list and near entries, deepest stack)
+// statistics (entries, tiles, decisions, list and near entries, longest queue)
 // are collected by their own instances of the forward kernel (kStats), so that
 // the others carry none of that bookkeeping; the adjoint collects none.
-template <bool kFp64, bool kStats>
+template <bool kFp64, bool kStats, bool kTeam>
 const void *forward_kernel(int damping, bool pot) {
     if constexpr (!kFp64) {
         (void)pot;
-        return damping ? (const void *)k_walk<false, true, false, false, kStats>
-                       : (const void *)k_walk<false, false, false, false, kStats>;
+        return damping ? (const void *)k_walk<false, true, false, false, kStats, kTeam>
+                       : (const void *)k_walk<false, false, false, false, kStats, kTeam>;
     } else {
         if (damping)
-            return pot ? (const void *)k_walk<true, true, true, false, kStats>
-                       : (const void *)k_walk<true, true, false, false, kStats>;
-        return pot ? (const void *)k_walk<true, false, true, false, kStats>
-                   : (const void *)k_walk<true, false, false, false, kStats>;
+            return pot ? (const void *)k_walk<true, true, true, false, kStats, kTeam>
+                       : (const void *)k_walk<true, true, false, false, kStats, kTeam>;
+        return pot ? (const void *)k_walk<true, false, true, false, kStats, kTeam>
+                   : (const void *)k_walk<true, false, false, false, kStats, kTeam>;
     }
 }
 
-const void *any_walk_kernel(bool fp64, bool adj, int damping, bool pot, bool stats) {
+template <bool kTeam>
+const void *walk_kernel(bool fp64, bool adj, int damping, bool pot, bool stats) {
     if (adj) {
-        if (fp64) return damping ? (const void *)k_walk<true, true, false, true, false> : (const void *)k_walk<true, false, false, true, false>;
-        return damping ? (const void *)k_walk<false, true, false, true, false> : (const void *)k_walk<false, false, false, true, false>;
+        if (fp64)
+            return damping ? (const void *)k_walk<true, true, false, true, false, kTeam>
+                           : (const void *)k_walk<true, false, false, true, false, kTeam>;
+        return damping ? (const void *)k_walk<false, true, false, true, false, kTeam>
+                       : (const void *)k_walk<false, false, false, true, false, kTeam>;
     }
-    if (fp64) return stats ? forward_kernel<true, true>(damping, pot) : forward_kernel<true, false>(damping, pot);
-    return stats ? forward_kernel<false, true>(damping, pot) : forward_kernel<false, false>(damping, pot);
+    if (fp64) return stats ? forward_kernel<true, true, kTeam>(damping, pot) : forward_kernel<true, false, kTeam>(damping, pot);
+    return stats ? forward_kernel<false, true, kTeam>(damping, pot) : forward_kernel<false, false, kTeam>(damping, pot);
+}
+
+const void *any_walk_kernel(bool team, bool fp64, bool adj, int damping, bool pot, bool stats) {
+    return team ? walk_kernel<true>(fp64, adj, damping, pot, stats) : walk_kernel<false>(fp64, adj, damping, pot, stats);
+}
+
+// No instance needs more dynamic shared memory than a launch gets without asking.
+constexpr size_t kPlainSmem = 48 << 10;
+static_assert(sizeof(SoloSmem<true, true>) * kWalkMaxWarps <= kPlainSmem && sizeof(SoloSmem<true, false>) * kWalkMaxWarps <= kPlainSmem &&
+                  sizeof(SoloSmem<false, true>) * kWalkMaxWarps <= kPlainSmem && sizeof(SoloSmem<false, false>) * kWalkMaxWarps <= kPlainSmem &&
+                  sizeof(TeamSmem<true, true>) <= kPlainSmem && sizeof(TeamSmem<true, false>) <= kPlainSmem &&
+                  sizeof(TeamSmem<false, true>) <= kPlainSmem && sizeof(TeamSmem<false, false>) <= kPlainSmem,
+              "larger ones need cudaFuncAttributeMaxDynamicSharedMemorySize");
+
+size_t solo_smem(bool fp64, bool adj) {
+    if (fp64) return adj ? sizeof(SoloSmem<true, true>) : sizeof(SoloSmem<true, false>);
+    return adj ? sizeof(SoloSmem<false, true>) : sizeof(SoloSmem<false, false>);
+}
+size_t team_smem(bool fp64, bool adj) {
+    if (fp64) return adj ? sizeof(TeamSmem<true, true>) : sizeof(TeamSmem<true, false>);
+    return adj ? sizeof(TeamSmem<false, true>) : sizeof(TeamSmem<false, false>);
+}
+
+cudaError_t launch(const void *k, const WalkArgs &a, unsigned blocks, unsigned warps, size_t smem, cudaStream_t st) {
+    WalkArgs args = a;
+    void *params[] = {&args};
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(blocks);
+    cfg.blockDim = dim3(warps * 32);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelExC(&cfg, k, params);
 }
 
 }  // namespace
 
-constexpr size_t kLargestWarpSmem =
-    sizeof(WarpSmem<true>) > sizeof(WarpSmem<false>) ? sizeof(WarpSmem<true>) : sizeof(WarpSmem<false>);
-
 // The grid is sized by the forward walk's instances. The adjoint's FP64 ones take
-// more registers (138-152 against 94-96): fewer of their blocks are resident, and
-// the rest start as those end and find the work counter drained (the walk waits on
-// nothing). Sizing every launch by the largest instance kept the FP64 forward walk
-// at 3 resident blocks of the 5 that fit: 1.295 -> 1.161 ms (sphere of 60,001,
-// damped), 2.27 -> 1.76 ms (sphere of 200,000).
+// more registers: fewer of their blocks are resident, and the rest start as those
+// end and find the work counter drained (groups wait for nothing). Sizing every
+// launch by the largest instance kept the FP64 forward walk at 3 resident blocks of
+// the 5 that fit: 1.295 -> 1.161 ms (sphere of 60,001, damped).
 cudaError_t walk_max_blocks_per_sm(bool fp64, unsigned warps, int *out) {
-    const size_t smem = (fp64 ? sizeof(WarpSmem<true>) : sizeof(WarpSmem<false>)) * warps;
     int minblocks = 1 << 30;
-    for (int q = 0; q < 16; q++) {
-        const bool adj = q & 1, damp = q & 2, pot = q & 4, stats = q & 8;
-        if (adj && (pot || stats)) continue;
-        const void *k = any_walk_kernel(fp64, adj, damp, pot, stats);
-        cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             (int)(kLargestWarpSmem * kWalkMaxWarps));
-        if (e != cudaSuccess) return e;
-        if (adj) continue;
+    for (int q = 0; q < 8; q++) {
+        const bool damp = q & 1, pot = q & 2, stats = q & 4;
+        if (pot && !fp64) continue;
         int nb = 0;
-        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k, (int)warps * 32, smem);
+        const cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(
+            &nb, any_walk_kernel(false, fp64, false, damp, pot, stats), (int)warps * 32, solo_smem(fp64, false) * warps);
         if (e != cudaSuccess) return e;
         minblocks = nb < minblocks ? nb : minblocks;
     }
@@ -1027,28 +1210,19 @@ cudaError_t walk_launch_shape(bool fp64, int device, unsigned warps, unsigned bl
     const int per_sm = blocks_per_sm ? (int)blocks_per_sm < maxb ? (int)blocks_per_sm : maxb : maxb;
     out->blocks = (unsigned)(sms * per_sm);
     out->warps = warps;
-    out->smem = (fp64 ? sizeof(WarpSmem<true>) : sizeof(WarpSmem<false>)) * warps;
+    out->sms = (unsigned)sms;
     return cudaSuccess;
 }
 
 cudaError_t launch_walk(const WalkArgs &a, bool fp64, const WalkLaunch &l, cudaStream_t st) {
-    const void *k = any_walk_kernel(fp64, a.adjoint != 0, a.damping, a.pot != nullptr, a.stats != 0);
-    unsigned blocks = l.blocks;
+    const bool adj = a.adjoint != 0;
+    const bool team = a.n_groups <= team_groups_per_sm(fp64, adj) * l.sms && a.t.n >= kTeamMinSize * a.systems;
+    const void *k = any_walk_kernel(team, fp64, adj, a.damping, a.pot != nullptr, a.stats != 0);
+    if (team)  // one block per group, as many as fit; the rest take the groups left
+        return launch(k, a, a.n_groups < kTeamBlocksPerSm * l.sms ? a.n_groups : kTeamBlocksPerSm * l.sms, kTeamMaxWarps,
+                      team_smem(fp64, adj), st);
     const unsigned need = (a.n_groups + l.warps - 1) / l.warps;
-    if (need < blocks) blocks = need ? need : 1;
-    WalkArgs args = a;
-    void *params[] = {&args};
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(blocks);
-    cfg.blockDim = dim3(l.warps * 32);
-    cfg.dynamicSmemBytes = l.smem;
-    cfg.stream = st;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    return cudaLaunchKernelExC(&cfg, k, params);
+    return launch(k, a, need < l.blocks ? need : l.blocks, l.warps, solo_smem(fp64, adj) * l.warps, st);
 }
 
 }  // namespace nbody

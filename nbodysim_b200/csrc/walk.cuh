@@ -7,13 +7,32 @@ namespace nbody {
 
 constexpr int kWalkWarps = 4;       // default warps per block (the autotuner may pick 1 or 2)
 constexpr int kWalkMaxWarps = 4;    // largest block the walk kernel is compiled for
-constexpr int kStackCap = 640;      // shared-memory stack entries per warp
-constexpr int kSpillChunk = kStackCap / 2;
-// A tile pushes at most 32 lanes x 8 children; after a spill the stack must
-// still have room for all of them.
-static_assert(kStackCap - kSpillChunk >= 32 * 8, "a spill must leave room for one tile's pushes");
-constexpr int kListFlush = 32;      // force pass once the interaction list holds this many
-constexpr int kListCap = kListFlush + 32;
+constexpr int kTeamMaxWarps = 4;    // warps of a block that walk one group together
+// Queue of the nodes a walk has still to examine (per warp in global memory, per
+// team in shared memory). Up to kQueueWide entries the oldest go first; beyond, the
+// newest, in tiles that get narrower until a depth-first descent of one entry at a
+// time (at most 7 more entries per level) fits in the reserve.
+constexpr uint32_t kQueueCap = 2048;
+constexpr uint32_t kQueueWide = 1280;
+constexpr uint32_t kQueueReserve = 7 * (kMaxLevels + 1) + 8;
+static_assert((kQueueCap & (kQueueCap - 1)) == 0, "ring index");
+static_assert(kQueueWide + 8 * 32 <= kQueueCap - kQueueReserve, "a tile's pushes fit before tiles get narrower");
+// Interaction lists: less than a batch of 32 left over, and what a tile (a team's tiles) adds.
+constexpr int kSoloList = 64;
+constexpr int kTeamList = 32 + 32 * kTeamMaxWarps;
+// Teams walk while there are at most this many groups per SM. Fewer groups leave
+// walk warps idle, and time is the chain of one group's tiles; with more, barriers
+// cost more than the last wave of single warps. Walk times, team against single
+// warps (us): MIXED 5000 particles 51 / 103, shell of 20,011 50 / 89, cubes of 48,000
+// 170 / 197, 56,000 195 / 206 and 70,000 240 / 228; its adjoint 5000 89 / 183, 85,000
+// 578 / 598, 100,000 682 / 648; FP64 5000 135 / 375, 16,384 226 / 580, 60,001 885 /
+// 1168, 112,000 1006 / 1235; its adjoint 16,384 310 / 671, 100,000 1460 / 1591.
+// Systems of fewer than kTeamMinSize particles have a few short tiles per group, for
+// which the barriers cost more (a step of 97: 133 us with teams, 125 without; 150:
+// the same; 300: 147 and 151).
+constexpr uint32_t kTeamMinSize = 160;
+constexpr unsigned team_groups_per_sm(bool fp64, bool adjoint) { return fp64 ? 24 : adjoint ? 16 : 12; }
+constexpr unsigned kTeamBlocksPerSm = 5;  // resident: 96 registers, ~36 KB of shared memory
 
 struct WalkArgs {
     Tree t;
@@ -26,9 +45,9 @@ struct WalkArgs {
     double *accd;       // FP64: user order, 3 doubles per particle
     uint32_t *counts;   // optional: accepted nodes per particle (user order)
     double *pot;        // optional: potential phi_i per particle (user order)
-    int2 *spill;        // per-warp spill regions (grid warps x spill_cap)
-    uint32_t spill_cap;
+    int2 *queue;        // kQueueCap entries per warp of the grid (walks by one warp)
     uint32_t n_groups;  // ceil(n / 32)
+    uint32_t systems;   // independent systems (1: a single one)
     int track_max_acc;  // reduce max |a| (adaptive dt)
     int stats;          // collect the walk statistics (DevScalars walk_* and max_stack)
     // Adjoint mode (frozen decisions): the walk computes, for the cotangent
@@ -52,11 +71,11 @@ struct WalkArgs {
 };
 
 // Launch shape of the persistent walk: `warps` per block, `blocks` in the grid
-// (a whole number of resident blocks per SM), `smem` bytes per block.
+// (a whole number of resident blocks per SM) of `sms` SMs.
 struct WalkLaunch {
     unsigned blocks;
     unsigned warps;
-    size_t smem;
+    unsigned sms;
 };
 // blocks_per_sm = 0: as many as fit. Returns the shape for that block size.
 cudaError_t walk_launch_shape(bool fp64, int device, unsigned warps, unsigned blocks_per_sm, WalkLaunch *out);

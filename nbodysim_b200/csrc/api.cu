@@ -114,15 +114,15 @@ struct nbody_ctx {
     // while the state drifts: they sort by the deepest split (sort_deep_p1, p2).
     int sort_deep_p1 = 8, sort_deep_p2 = 8;
     bool multi_step_call = false;
+    // The same for several systems (TreeBuild::sort_pm; 0: the full sort).
+    int sort_pm = 0, sort_deep_pm = 0, sort_pm_cooldown = 0;
+    int sys_bits = 1;  // bits of a system's number
     // CUDA graphs: one captured step replayed per step; per-offset graphs for the
     // adjoint's recompute and reverse steps. Rebuilt when their key changes.
     bool use_graphs = true;
     std::vector<unsigned char> step_key, adj_key;
     cudaGraphExec_t step_exec = nullptr;
     unsigned step_launches = 0;
-    unsigned step_cond_launches = 0;  // of those, the kernels of the full sort's conditional node
-    unsigned capture_cond_launches = 0;
-    unsigned replayed_cond_launches = 0;  // of the last replayed step, added if its full sort ran
     std::vector<cudaGraphExec_t> rec_exec, adj_exec;
     std::vector<unsigned> rec_launches, adj_launches;
     // image rendering buffers (grown on demand)
@@ -141,8 +141,6 @@ struct nbody_ctx {
     size_t direct_bytes = 0;
     // nbody_step_host: masses and velocities uploaded on a second stream while the tree is built
     cudaStream_t aux_stream = nullptr;
-    // captures the tree build's full sort into a conditional graph node
-    cudaStream_t cond_stream = nullptr;
     cudaEvent_t ev_fork = nullptr, ev_mass = nullptr, ev_vel = nullptr;
     cudaEvent_t mass_pending = nullptr;  // set while a force pass must wait for ev_mass before reading masses
 };
@@ -278,6 +276,32 @@ void next_sort_plan(nbody_ctx *c, const DevScalars &h) {
     }
 }
 
+// The next build's plan for several systems: passes over the top bits of the
+// system's number and the first word together (at most 8; what these leave tied is
+// sorted in place), by the rules above, or the full sort.
+void next_systems_plan(nbody_ctx *c, const DevScalars &h) {
+    if (h.max_prefix_bits == 0) return;
+    const uint32_t bits = h.max_prefix_bits + (uint32_t)c->sys_bits;
+    const uint64_t tol = std::max<uint64_t>(64, c->n / kTieShare);
+    uint64_t tied = h.pair_passes[kPassBins - 1];  // pairs that all 64 bits leave tied
+    const int covered = bits <= 64 ? (int)(bits + 7) / 8 : 0;
+    if (h.word_ties) c->sort_pm_cooldown = kPlanCooldown;
+    int want = covered ? covered : c->sort_pm_cooldown == 0 && tied <= tol ? 8 : 0;
+    if (c->sort_pm_cooldown == 0) {
+        while (want > 1) {
+            tied += h.pair_passes[want];
+            if (tied > tol) break;
+            want--;
+        }
+    }
+    if (c->sort_pm_cooldown > 0) c->sort_pm_cooldown--;
+    auto follow = [&](int &plan, int to, bool always) {
+        if (always || to == 0 || plan == 0 || to > plan || plan - to >= 2) plan = to;
+    };
+    follow(c->sort_pm, want, h.word_ties);
+    follow(c->sort_deep_pm, covered, h.word_ties || h.tie_runs);
+}
+
 // Marks an API call of several steps for its duration (tree_inputs picks the
 // deepest-split sort plan).
 struct MultiStepCall {
@@ -298,8 +322,6 @@ int check_status(nbody_ctx *c) {
     s.walk_decisions = h.walk_decisions;
     s.walk_list = h.walk_list;
     s.walk_near = h.walk_near;
-    if (h.word_ties) c->launches += c->replayed_cond_launches;  // the replayed step ran its full sort
-    c->replayed_cond_launches = 0;
     s.kernel_launches = c->launches;
     {
         const WalkLaunch &w = c->p.precision == NBODY_PRECISION_FP64 ? c->wl_fp64 : c->wl_mixed;
@@ -316,12 +338,19 @@ int check_status(nbody_ctx *c) {
     s.last_dt = h.dt_used;
     for (int k = 0; k < 3; k++) s.root_center[k] = h.root_center[k];
     s.root_side = h.root_side;
-    const int used_plan = c->multi_step_call ? c->sort_deep_p1 + c->sort_deep_p2 : c->sort_p1 + c->sort_p2;
-    s.sort_passes = c->nsys > 1 ? 18u : (uint32_t)used_plan + (h.word_ties ? 16u : 0u);
     s.sort_split_bits = h.max_prefix_bits;
     s.sort_tie_runs = h.tie_runs;
-    next_sort_plan(c, h);
-    s.sort_next_passes = c->nsys > 1 ? 18u : (uint32_t)(c->sort_p1 + c->sort_p2);
+    if (c->tb.nsys > 1) {
+        const int used = c->multi_step_call ? c->sort_deep_pm : c->sort_pm;
+        s.sort_passes = used == 0 ? 18u : (uint32_t)used + (h.word_ties ? 18u : 0u);
+        next_systems_plan(c, h);
+        s.sort_next_passes = c->sort_pm == 0 ? 18u : (uint32_t)c->sort_pm;
+    } else {
+        const int used = c->multi_step_call ? c->sort_deep_p1 + c->sort_deep_p2 : c->sort_p1 + c->sort_p2;
+        s.sort_passes = (uint32_t)used + (h.word_ties ? 16u : 0u);
+        next_sort_plan(c, h);
+        s.sort_next_passes = (uint32_t)(c->sort_p1 + c->sort_p2);
+    }
     if (c->timing) {
         float ms[4] = {0, 0, 0, 0};
         for (int k = 0; k < 4; k++) cudaEventElapsedTime(&ms[k], c->ev[k], c->ev[k + 1]);
@@ -347,9 +376,9 @@ void tree_inputs(nbody_ctx *c, uint32_t n, bool want_vmax) {
     tb.single = single(c) ? 1 : 0;
     tb.sort_p1 = c->multi_step_call ? c->sort_deep_p1 : c->sort_p1;
     tb.sort_p2 = c->multi_step_call ? c->sort_deep_p2 : c->sort_p2;
-    tb.sort_checked = 1;
-    tb.cond_stream = c->cond_stream;
-    tb.cond_launches = &c->capture_cond_launches;
+    tb.sort_pm = c->multi_step_call ? c->sort_deep_pm : c->sort_pm;
+    tb.sys_bits = c->sys_bits;
+    tb.reset = 0;
 }
 
 void ev(nbody_ctx *c, int k) {
@@ -365,8 +394,7 @@ int force_pass(nbody_ctx *c, int damping, double theta, bool fp64, bool want_vma
                const WalkLaunch *shape = nullptr, bool min_size = false, int save_slot = -1, int restore_slot = -1,
                double *acc64_out = nullptr) {
     uint32_t n = c->n;
-    unsigned launches = 1;
-    NB_CUDA(launch_reset_pass(c->sc, c->stream));
+    unsigned launches = 0;
     tree_inputs(c, n, want_vmax);
     if (pos) c->tb.pos = pos;
     const bool multi = c->nsys > 1 && !c->single_pass && c->sys_total == n;
@@ -379,10 +407,13 @@ int force_pass(nbody_ctx *c, int damping, double theta, bool fp64, bool want_vma
     ev(c, 0);
     if (restore_slot >= 0 && !multi) {
         // the octree of these positions was saved by the forward recomputation
+        NB_CUDA(launch_reset_pass(c->sc, c->stream));
+        launches++;
         int rc = copy_tree_slot(c, (uint32_t)restore_slot, false);
         if (rc) return rc;
         ev(c, 1);
     } else {
+        c->tb.reset = 1;
         NB_CUDA(build_octree(c->tb, c->stream, &launches));
         if (min_size && c->p.min_node_size > 0 && n >= 2 && !multi) {
             int rc = apply_min_size(c, want_vmax, &launches);
@@ -484,7 +515,7 @@ int download_acc(nbody_ctx *c, double *acc) {
 std::vector<unsigned char> graph_key(nbody_ctx *c, uint32_t extra) {
     struct K {
         uint32_t n, nsys, ngroups, extra;
-        int sort_p1, sort_p2, walk_stats;
+        int sort_p1, sort_p2, sort_pm, walk_stats;
         void *arena, *adj, *sys, *stream;
         nbody_params p;
         WalkLaunch wm, wf;
@@ -492,7 +523,9 @@ std::vector<unsigned char> graph_key(nbody_ctx *c, uint32_t extra) {
     std::memset(&k, 0, sizeof k);
     k.n = c->n; k.nsys = c->nsys; k.ngroups = c->ngroups; k.extra = extra;
     k.sort_p1 = c->multi_step_call ? c->sort_deep_p1 : c->sort_p1;
-    k.sort_p2 = c->multi_step_call ? c->sort_deep_p2 : c->sort_p2; k.walk_stats = c->walk_stats;
+    k.sort_p2 = c->multi_step_call ? c->sort_deep_p2 : c->sort_p2;
+    k.sort_pm = c->multi_step_call ? c->sort_deep_pm : c->sort_pm;
+    k.walk_stats = c->walk_stats;
     k.arena = c->arena; k.adj = c->adj_arena; k.sys = c->sys_arena; k.stream = (void *)c->stream;
     k.p = c->p; k.wm = c->wl_mixed; k.wf = c->wl_fp64;
     const unsigned char *b = (const unsigned char *)&k;
@@ -724,17 +757,13 @@ int run_steps(nbody_ctx *c, uint32_t nsteps) {
         if (!c->step_exec || key != c->step_key) {
             drop_graph(c->step_exec);
             c->step_key.clear();
-            c->capture_cond_launches = 0;
             if (capture(c, &c->step_exec, &c->step_launches, [&] { return one_step(c); })) c->step_key = key;
-            c->step_cond_launches = c->capture_cond_launches;
         }
         if (c->step_exec) {
-            // the conditional node's kernels are counted when a replay ran them (check_status)
             for (uint32_t s = 0; s < nsteps; s++) {
                 NB_CUDA(cudaGraphLaunch(c->step_exec, c->stream));
-                c->launches += c->step_launches - c->step_cond_launches;
+                c->launches += c->step_launches;
             }
-            c->replayed_cond_launches = c->step_cond_launches;
             return NBODY_OK;
         }
     }
@@ -998,8 +1027,6 @@ int nbody_create(const nbody_params *p, nbody_ctx **out) {
     if (cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking) != cudaSuccess)
         return cleanup(fail(NBODY_ERR_CUDA, "stream creation failed%s"));
     c->own_stream = true;
-    if (cudaStreamCreateWithFlags(&c->cond_stream, cudaStreamNonBlocking) != cudaSuccess)
-        return cleanup(fail(NBODY_ERR_CUDA, "stream creation failed%s"));
     if (cudaMalloc(&c->sc, sizeof(DevScalars)) != cudaSuccess) return cleanup(fail(NBODY_ERR_OOM, "scalars%s"));
     if (cudaMemset(c->sc, 0, sizeof(DevScalars)) != cudaSuccess) return cleanup(fail(NBODY_ERR_CUDA, "memset%s"));
     if (cudaMallocHost(&c->hsc, sizeof(DevScalars)) != cudaSuccess) return cleanup(fail(NBODY_ERR_OOM, "pinned%s"));
@@ -1038,7 +1065,6 @@ int nbody_destroy(nbody_ctx *c) {
     if (c->pairs) cudaFree(c->pairs);
     if (c->hcounters) cudaFreeHost(c->hcounters);
     if (c->aux_stream) cudaStreamDestroy(c->aux_stream);
-    if (c->cond_stream) cudaStreamDestroy(c->cond_stream);
     if (c->ev_fork) cudaEventDestroy(c->ev_fork);
     if (c->ev_mass) cudaEventDestroy(c->ev_mass);
     if (c->ev_vel) cudaEventDestroy(c->ev_vel);
@@ -1179,6 +1205,9 @@ int nbody_set_systems(nbody_ctx *c, uint32_t nsys, const uint32_t *counts) {
     c->nsys = nsys;
     c->sys_total = (uint32_t)total;
     c->ngroups = ngroups;
+    c->sys_bits = 1;
+    while (c->sys_bits < 16 && ((nsys - 1) >> c->sys_bits)) c->sys_bits++;
+    c->sort_pm = c->sort_deep_pm = c->sort_pm_cooldown = 0;
     return NBODY_OK;
 }
 

@@ -65,9 +65,12 @@ enum : uint32_t {
 
 // Pairs of neighbouring keys are binned by the sort passes that separate them:
 // 1-8 passes cover the first 63-bit key word, 9-16 also the second; bin 17 is a
-// pair equal over both words.
+// pair equal over both words. With several systems the first word follows the
+// system's number (sys_bits) in a 64-bit key: 1-8 passes cover the key, bin 17 is a
+// pair equal over it.
 constexpr int kPassBins = 18;
-__host__ __device__ inline int passes_for_bits(uint32_t bits) {
+__host__ __device__ inline int passes_for_bits(uint32_t bits, uint32_t sys_bits = 0) {
+    if (sys_bits) return bits + sys_bits <= 64 ? (int)(bits + sys_bits + 7) / 8 : kPassBins - 1;
     return bits <= 63 ? (int)(bits + 7) / 8 : bits <= 126 ? 8 + (int)(bits - 63 + 7) / 8 : kPassBins - 1;
 }
 
@@ -107,6 +110,31 @@ struct DevScalars {
     double lam_scale;
     double diag[16];          // kinetic, potential, momentum[3], L[3], mass, m*x[3]
 };
+
+// Starting values of a force pass (the status bits and the call's totals stay).
+__device__ inline void reset_pass(DevScalars *sc) {
+    sc->interactions = 0;
+    sc->walk_entries = 0;
+    sc->walk_tiles = 0;
+    sc->walk_decisions = 0;
+    sc->walk_list = 0;
+    sc->walk_near = 0;
+    sc->n_onodes = 0;
+    sc->depth = 0;
+    sc->max_stack = 0;
+    sc->fallback_tests = 0;
+    sc->group_counter = 0;
+    sc->ticket = 0;
+    sc->deep_groups = 0;
+    sc->word_ties = 0;
+    sc->tie_runs = 0;
+    sc->max_prefix_bits = 0;
+    for (int k = 0; k < kPassBins; k++) sc->pair_passes[k] = 0;
+    sc->max_acc_bits = 0;
+    sc->max_vel_bits = 0;
+}
+// The same as a launch of its own, for passes that build no octree (step.cu).
+cudaError_t launch_reset_pass(DevScalars *sc, cudaStream_t st);
 
 struct Tree {
     uint32_t n;

@@ -108,25 +108,7 @@ __global__ void k_diag(const double *__restrict__ pos, const double *__restrict_
 
 __global__ void k_reset_pass(DevScalars *sc) {
     griddep();
-    sc->interactions = 0;
-    sc->walk_entries = 0;
-    sc->walk_tiles = 0;
-    sc->walk_decisions = 0;
-    sc->walk_list = 0;
-    sc->walk_near = 0;
-    sc->n_onodes = 0;
-    sc->depth = 0;
-    sc->max_stack = 0;
-    sc->fallback_tests = 0;
-    sc->group_counter = 0;
-    sc->ticket = 0;
-    sc->deep_groups = 0;
-    sc->word_ties = 0;
-    sc->tie_runs = 0;
-    sc->max_prefix_bits = 0;
-    for (int k = 0; k < kPassBins; k++) sc->pair_passes[k] = 0;
-    sc->max_acc_bits = 0;
-    sc->max_vel_bits = 0;
+    reset_pass(sc);
 }
 
 __global__ void k_acc_to_double(const float *__restrict__ in, double *__restrict__ out, size_t count) {

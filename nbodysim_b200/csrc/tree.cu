@@ -8,6 +8,7 @@
 // emulated below, the same centre of mass as their bottom node, so every
 // particle's walk accepts the same bodies (see walk.cu).
 #include "tree.cuh"
+#include "keys.cuh"
 #include "sort.cuh"
 
 #include <cstdio>
@@ -47,9 +48,16 @@ __device__ inline void root_from_extrema(const double *lo, const double *hi, boo
 // Root cube (root_from_extrema) over all particles. Also flags
 // non-finite positions (masses are checked where the bodies are gathered), and
 // (optionally) reduces max |v| for the adaptive step.
+// The first kernel of a build, so it also zeroes the sort's counters and, with
+// reset, gives the pass's scalars their starting values. Those two, the digit counts
+// (k_keys), their scan (each sort tile) and the full sort's 22 were launches of their
+// own: a step of 97 particles 130 -> 114 us, of 5000 212 -> 191 us.
 __global__ void k_bbox(const double *__restrict__ pos, const double *__restrict__ vel, uint32_t n,
-                       double *__restrict__ partial, DevScalars *sc, int keep_root, int single) {
+                       double *__restrict__ partial, DevScalars *sc, int keep_root, int single,
+                       uint4 *__restrict__ zero, size_t zero_quads, int reset) {
     griddep();
+    for (size_t i = blockIdx.x * blockDim.x + threadIdx.x; i < zero_quads; i += (size_t)gridDim.x * blockDim.x)
+        zero[i] = make_uint4(0u, 0u, 0u, 0u);
     __shared__ double s_red[7][32];
     __shared__ bool s_last;
     double mn[3] = {INFINITY, INFINITY, INFINITY};
@@ -108,6 +116,7 @@ __global__ void k_bbox(const double *__restrict__ pos, const double *__restrict_
     double r[7];
 #pragma unroll
     for (int k = 0; k < 7; k++) r[k] = warp_min(lane < nw ? s_red[k][lane] : INFINITY);
+    if (lane == 0 && reset) reset_pass(sc);
     if (lane == 0 && keep_root) {
         sc->max_vel_bits = (unsigned long long)__double_as_longlong(sqrt(-r[6]));
         sc->ticket = 0;
@@ -161,95 +170,64 @@ __global__ void k_bbox_systems(const double *__restrict__ pos, const double *__r
 }
 
 // ---------------------------------------------------------------------------
-// Octant digits by descent from the root cube, rounding every child centre
-// exactly as allocate_child does (src/octree.cpp:65-84: center + (+-1 * half) / 2
-// with half = side / 2), and choosing the octant with strict '>' as
-// add_particle does (src/octree.cpp:153-165). Digits are (z<<2)|(y<<1)|x so
-// that Morton order equals the reference's child order 0..7. T is the
-// reference build's datatype: double, or float for its FLOAT build.
-__device__ inline double add_rn(double a, double b) { return __dadd_rn(a, b); }
-__device__ inline float add_rn(float a, float b) { return __fadd_rn(a, b); }
-
-template <typename T>
-__device__ inline uint64_t descend_word(T x, T y, T z, T &cx, T &cy, T &cz, T &side) {
-    uint64_t key = 0;
-#pragma unroll 3
-    for (int l = 0; l < kLevelsPerWord; l++) {
-        const T half = side / T(2);
-        const T q = half / T(2);
-        int bx = x > cx, by = y > cy, bz = z > cz;
-        key = (key << 3) | (uint64_t)((bz << 2) | (by << 1) | bx);
-        cx = add_rn(cx, bx ? q : -q);
-        cy = add_rn(cy, by ? q : -q);
-        cz = add_rn(cz, bz ? q : -q);
-        side = half;
-    }
-    return key;
-}
-
-// `words` key words of one particle from the root cube (center, side).
-template <typename T>
-__device__ inline void descend_words(const double *p, const double *root, int words, uint64_t *out) {
-    T cx = (T)root[0], cy = (T)root[1], cz = (T)root[2], s = (T)root[3];
-    const T x = (T)p[0], y = (T)p[1], z = (T)p[2];
-    for (int w = 0; w < words; w++) out[w] = descend_word<T>(x, y, z, cx, cy, cz, s);
-}
-
 // Key words per particle: levels 1..21 (k1) and 22..42 (k2). Escaped
 // particles can make the root cube many orders of magnitude larger than the
 // bulk of the system, so the first 21 levels alone do not separate it. With
 // k2_user null only k1 is computed (a sort plan that needs no second word).
-// The sort key (k1 or k2) goes to `sortkey`, the identity to `idx`.
-__global__ void k_keys(const double *__restrict__ pos, uint32_t n, const DevScalars *sc,
-                       uint64_t *__restrict__ k1_user, uint64_t *__restrict__ sortkey,
-                       uint64_t *__restrict__ k2_user, uint32_t *__restrict__ idx,
-                       const uint32_t *__restrict__ sys_id, const double *__restrict__ sys_root, int single,
-                       int sort_by_k1) {
+// The sort key goes to `sortkey`, the identity to `idx`: the second word, or
+// without it the first, or with sys_id the system's number (sys_bits) above the
+// first word's top bits. The digits of the sort's passes are counted on the way,
+// per block in shared memory: `passes` of the sort key (shift of the first one:
+// `shift`) into slots 0.. and, with k2_user, the 8 of k1 into slots 8...
+__global__ void __launch_bounds__(256)
+    k_keys(const double *__restrict__ pos, uint32_t n, const DevScalars *sc, uint64_t *__restrict__ k1_user,
+           uint64_t *__restrict__ sortkey, uint64_t *__restrict__ k2_user, uint32_t *__restrict__ idx,
+           const uint32_t *__restrict__ sys_id, const double *__restrict__ sys_root, int sys_bits, int single,
+           int passes, int shift, uint32_t *__restrict__ hist) {
     griddep();
-    uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    double root[4];
-    if (sys_id) {
-        const double *r = sys_root + 4 * (size_t)sys_id[i];
-        root[0] = r[0]; root[1] = r[1]; root[2] = r[2]; root[3] = r[3];
-    } else {
+    __shared__ uint32_t s_h[16 * 256];
+    const int both = k2_user ? 8 : 0, words = k2_user ? 2 : 1;
+    for (int k = threadIdx.x; k < (both ? 16 : passes) * 256; k += blockDim.x) s_h[k] = 0u;
+    __syncthreads();
+    double root[4] = {0.0, 0.0, 0.0, 0.0};
+    if (!sys_id) {
         root[0] = sc->root_center[0]; root[1] = sc->root_center[1]; root[2] = sc->root_center[2];
         root[3] = sc->root_side;
     }
-    const double p[3] = {pos[3 * (size_t)i], pos[3 * (size_t)i + 1], pos[3 * (size_t)i + 2]};
-    const int words = k2_user ? 2 : 1;
-    uint64_t w[2] = {0, 0};
-    if (single) descend_words<float>(p, root, words, w);
-    else descend_words<double>(p, root, words, w);
-    k1_user[i] = w[0];
-    sortkey[i] = sort_by_k1 ? w[0] : w[1];
-    if (k2_user) k2_user[i] = w[1];
-    idx[i] = i;
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        uint64_t sys = 0;
+        if (sys_id) {
+            sys = sys_id[i];
+            const double *r = sys_root + 4 * (size_t)sys;
+            root[0] = r[0]; root[1] = r[1]; root[2] = r[2]; root[3] = r[3];
+        }
+        const double p[3] = {pos[3 * (size_t)i], pos[3 * (size_t)i + 1], pos[3 * (size_t)i + 2]};
+        uint64_t w[2] = {0, 0};
+        if (single) descend_words<float>(p, root, words, w);
+        else descend_words<double>(p, root, words, w);
+        k1_user[i] = w[0];
+        const uint64_t key = sys_id ? (sys << (64 - sys_bits)) | (w[0] >> (sys_bits - 1)) : k2_user ? w[1] : w[0];
+        sortkey[i] = key;
+        if (k2_user) k2_user[i] = w[1];
+        idx[i] = i;
+        for (int q = 0; q < passes; q++) atomicAdd(&s_h[q * 256 + ((key >> (shift + 8 * q)) & 255u)], 1u);
+        for (int q = 0; q < both; q++) atomicAdd(&s_h[(8 + q) * 256 + ((w[0] >> (8 * q)) & 255u)], 1u);
+    }
+    __syncthreads();
+    for (int k = threadIdx.x; k < (both ? 16 : passes) * 256; k += blockDim.x)
+        if (s_h[k]) atomicAdd(&hist[k], s_h[k]);
 }
 
-// The second key words (single system), for a full sort that follows a plan
-// without them; nothing unless *run_if is non-zero.
-__global__ void k_keys_second(const double *__restrict__ pos, uint32_t n, const DevScalars *sc,
-                              uint64_t *__restrict__ k2_user, int single, const uint32_t *run_if) {
-    griddep();
-    if (*run_if == 0u) return;
-    uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const double root[4] = {sc->root_center[0], sc->root_center[1], sc->root_center[2], sc->root_side};
-    const double p[3] = {pos[3 * (size_t)i], pos[3 * (size_t)i + 1], pos[3 * (size_t)i + 2]};
-    uint64_t w[2];
-    if (single) descend_words<float>(p, root, 2, w);
-    else descend_words<double>(p, root, 2, w);
-    k2_user[i] = w[1];
-}
-
-// dst[j] = src[idx[j]]; with run_if non-null, only when *run_if is non-zero.
+// dst[j] = src[idx[j]], and the systems likewise (sys_id null: none).
 __global__ void k_gather_key(const uint64_t *__restrict__ src, const uint32_t *__restrict__ idx,
-                             uint64_t *__restrict__ dst, uint32_t n, const uint32_t *run_if) {
+                             uint64_t *__restrict__ dst, uint32_t n, const uint32_t *__restrict__ sys_id,
+                             uint32_t *__restrict__ sys_sorted) {
     griddep();
-    if (run_if && *run_if == 0u) return;
     uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j < n) dst[j] = src[idx[j]];
+    if (j >= n) return;
+    const uint32_t i = idx[j];
+    dst[j] = src[i];
+    if (sys_id) sys_sorted[j] = sys_id[i];
 }
 
 // Runs of neighbours that the sort plan left equal over its bits, (k1 >> s1)
@@ -260,17 +238,19 @@ __global__ void k_gather_key(const uint64_t *__restrict__ src, const uint32_t *_
 // keep the user order as the full LSD sort keeps it. Runs are disjoint and a
 // permutation inside a run leaves every prefix of the run unchanged, so the
 // runs are found and sorted concurrently. A longer run sets the flag of the
-// full sort (inside a captured graph, the condition of its graph node).
+// full sort. Runs of several systems lie within one system.
 constexpr uint32_t kMaxTieRun = 64;
 
 __global__ void k_fix_ties(uint64_t *__restrict__ k1_sorted, uint64_t *__restrict__ k2_sorted,
                            uint32_t *__restrict__ idx, const double *__restrict__ pos, int have_k2, int s1, int s2,
-                           uint32_t n, int single, DevScalars *sc, cudaGraphConditionalHandle cond, int use_cond) {
+                           uint32_t n, int single, const uint32_t *__restrict__ sys,
+                           const double *__restrict__ sys_root, DevScalars *sc) {
     griddep();
     const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
     auto same = [&](uint32_t a, uint32_t b) {
         bool t = (k1_sorted[a] >> s1) == (k1_sorted[b] >> s1);
         if (t && have_k2) t = (k2_sorted[a] >> s2) == (k2_sorted[b] >> s2);
+        if (t && sys) t = sys[a] == sys[b];
         return t;
     };
     if (j + 1 >= n || !same(j, j + 1) || (j > 0 && same(j - 1, j))) return;  // not the first of a run
@@ -278,7 +258,6 @@ __global__ void k_fix_ties(uint64_t *__restrict__ k1_sorted, uint64_t *__restric
     while (e + 1 < n && same(e, e + 1)) {
         if (++e - j + 1 > kMaxTieRun) {
             atomicOr(&sc->word_ties, 1u);
-            if (use_cond) cudaGraphSetConditional(cond, 1u);
             return;
         }
     }
@@ -299,7 +278,11 @@ __global__ void k_fix_ties(uint64_t *__restrict__ k1_sorted, uint64_t *__restric
             k1_sorted[p] = a1;
             idx[p] = ai;
         }
-        const double root[4] = {sc->root_center[0], sc->root_center[1], sc->root_center[2], sc->root_side};
+        double root[4] = {sc->root_center[0], sc->root_center[1], sc->root_center[2], sc->root_side};
+        if (sys) {
+            const double *r = sys_root + 4 * (size_t)sys[j];
+            root[0] = r[0]; root[1] = r[1]; root[2] = r[2]; root[3] = r[3];
+        }
         for (uint32_t a = j; a < e;) {
             uint32_t b = a;
             while (b < e && k1_sorted[b + 1] == k1_sorted[a]) b++;
@@ -343,28 +326,6 @@ __global__ void k_fix_ties(uint64_t *__restrict__ k1_sorted, uint64_t *__restric
         k2_sorted[p] = a2;
         idx[p] = ai;
     }
-}
-
-// Start of the full sort after ties: the second words as sort keys, identity indices.
-__global__ void k_full_sort_init(const uint64_t *__restrict__ k2_user, uint64_t *__restrict__ key,
-                                 uint32_t *__restrict__ idx, uint32_t n, const uint32_t *run_if) {
-    griddep();
-    if (*run_if == 0u) return;
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) {
-        key[i] = k2_user[i];
-        idx[i] = i;
-    }
-}
-
-__global__ void k_gather_sys(const uint32_t *__restrict__ sys_id, const uint32_t *__restrict__ idx,
-                             uint64_t *__restrict__ key, uint32_t *__restrict__ sys_sorted, uint32_t n) {
-    griddep();
-    uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= n) return;
-    const uint32_t s = sys_id[idx[j]];
-    if (key) key[j] = s;
-    if (sys_sorted) sys_sorted[j] = s;
 }
 
 // Exclusive prefix sum of u32 values in place: tiles of 4096 scanned per
@@ -568,7 +529,8 @@ struct DeltaFrom {
 
 __global__ void k_radix_tree(KeyView kv, int32_t *__restrict__ bleft, int32_t *__restrict__ bright,
                              int32_t *__restrict__ bparent, int32_t *__restrict__ leaf_bparent,
-                             int32_t *__restrict__ bdelta, uint32_t *max_prefix_bits, uint32_t *pair_passes) {
+                             int32_t *__restrict__ bdelta, uint32_t *max_prefix_bits, uint32_t *pair_passes,
+                             uint32_t sys_bits) {
     __shared__ uint32_t hist[kPassBins];
     griddep();
     int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -583,7 +545,7 @@ __global__ void k_radix_tree(KeyView kv, int32_t *__restrict__ bleft, int32_t *_
     if (threadIdx.x < kPassBins) hist[threadIdx.x] = 0u;
     __syncthreads();
     {
-        const int bin = dn >= 0 ? passes_for_bits((uint32_t)dn + 1u) : -1;
+        const int bin = dn >= 0 ? passes_for_bits((uint32_t)dn + 1u, sys_bits) : -1;
         const uint32_t same = __match_any_sync(0xffffffffu, bin);
         if (bin >= 0 && (threadIdx.x & 31) == __ffs(same) - 1) atomicAdd(&hist[bin], (uint32_t)__popc(same));
     }
@@ -875,152 +837,104 @@ static inline unsigned blocks_for(uint64_t n, unsigned t) { return (unsigned)((n
 cudaError_t build_octree(const TreeBuild &tb, cudaStream_t st, unsigned *launches) {
     const uint32_t n = tb.n;
     unsigned L = 0;
-    if (n == 0) return cudaSuccess;
+    if (n == 0) return tb.reset ? launch_reset_pass(tb.sc, st) : cudaSuccess;
     const bool multi = tb.nsys > 1;
+    // The plan's passes: on the second word, on the first, or (several systems) on the
+    // system's number and the first word together.
+    const int p2 = multi ? 0 : tb.sort_p2, p1 = multi ? 0 : tb.sort_p1, pm = multi ? tb.sort_pm : 0;
+    const int passes_used = multi ? pm : p2 > 0 ? 8 + 8 : p1;
     // root cube (+ max |v| when requested); one per system when there are several
-    launch_pdl(k_bbox, dim3(tb.bbox_blocks), dim3(256), 0, st, tb.pos, tb.vel_for_max, n, tb.bbox_partial, tb.sc,
-                                           multi ? 0 : tb.keep_root, tb.single);
+    const unsigned bbox_blocks = std::max(1u, std::min(tb.bbox_blocks, blocks_for(n, 1024)));
+    launch_pdl(k_bbox, dim3(bbox_blocks), dim3(256), 0, st, tb.pos, tb.vel_for_max, n, tb.bbox_partial, tb.sc,
+               multi ? 0 : tb.keep_root, tb.single, reinterpret_cast<uint4 *>(tb.sort_scratch),
+               sort_zero_words(n, passes_used) / 4, tb.reset);
+    L += 1;
     if (multi) {
         if (tb.mass_ready) cudaStreamWaitEvent(st, tb.mass_ready, 0);
         launch_pdl(k_bbox_systems, dim3(tb.nsys), dim3(256), 0, st, tb.pos, tb.mass, tb.sys_start, tb.sys_root, tb.sc, tb.single);
         L += 1;
     }
-    uint32_t *sort_err = &tb.sc->status;
-    uint32_t *ties = &tb.sc->word_ties;
-    // `count` LSD passes with the digits of a `plan`-pass sort of one word
-    // (digit_shift), histogram and status slots from `slot`, ping-ponging
+    uint32_t *err = &tb.sc->status;
+    const uint32_t *sys_id = multi ? tb.sys_id : nullptr, *sys_sorted = multi ? tb.sys_sorted : nullptr;
+    // `count` LSD passes with shifts from `shift`, slots from `slot`, ping-ponging
     // (kin, iin) and (kout, iout): an even count leaves the result in (kin, iin),
     // an odd one in (kout, iout).
-    auto passes = [&](uint64_t *kin, uint64_t *kout, uint32_t *iin, uint32_t *iout, int count, int plan, int slot,
-                      const uint32_t *run_if, cudaStream_t s) {
+    auto passes = [&](uint64_t *kin, uint64_t *kout, uint32_t *iin, uint32_t *iout, int count, int shift, int slot) {
         for (int q = 0; q < count; q++) {
-            sort_pass(kin, iin, kout, iout, n, slot + q, digit_shift(plan, q), tb.sort_scratch, sort_err,
-                      kStatusSortStall, run_if, s, &L);
+            sort_pass(kin, iin, kout, iout, n, slot + q, shift + 8 * q, tb.sort_scratch, err, kStatusSortStall, st, &L);
             uint64_t *tk = kin; kin = kout; kout = tk;
             uint32_t *ti = iin; iin = iout; iout = ti;
         }
     };
-    auto gather = [&](const uint64_t *src, uint64_t *dst, const uint32_t *run_if, cudaStream_t s) {
-        launch_pdl(k_gather_key, dim3(blocks_for(n, 256)), dim3(256), 0, s, src, tb.idx_a, dst, n, run_if);
+    auto gather = [&](const uint64_t *src, uint64_t *dst, const uint32_t *sid) {
+        launch_pdl(k_gather_key, dim3(blocks_for(n, 256)), dim3(256), 0, st, src, tb.idx_a, dst, n, sid, tb.sys_sorted);
         L += 1;
     };
-    // Slots: passes on k2 0-7, on k1 8-15, on the system id 16-17; the full sort
-    // after a plan that left ties, k2 18-25 and k1 26-33.
+    auto keys = [&](uint64_t *sortkey, uint64_t *k2, uint32_t *idx, int count, int shift) {
+        launch_pdl(k_keys, dim3(std::min(1184u, blocks_for(n, 256))), dim3(256), 0, st, tb.pos, n, tb.sc, tb.key3, sortkey,
+                   k2, idx, sys_id, tb.sys_root, tb.sys_bits, tb.single, count, shift, tb.sort_scratch);
+        L += 1;
+    };
+    FullSort full{tb.key_a, tb.key_b, tb.key3, tb.key2, tb.idx_a, tb.idx_b, sys_id, tb.sys_sorted, n, tb.sort_scratch, err,
+                  kStatusSortStall, &tb.sc->word_ties, p2 > 0, tb.pos, tb.sc, tb.sys_root, tb.single};
     // Every plan leaves k1 in sorted order in key_b and the permutation in idx_a
     // (a plan with an odd pass count starts in the other buffers). The user-order
     // words: k1 in key3, k2 in key2.
-    const int p2 = multi ? 8 : tb.sort_p2, p1 = multi ? 8 : tb.sort_p1;
-    const bool checked = !multi && tb.sort_checked && !(p2 >= 8 && p1 >= 8);
-    if (p2 > 0) {
+    bool checked = true;
+    int s1 = 0, s2 = 0;  // the tie check's shifts of the first and second words
+    if (multi && pm == 0) {
+        keys(tb.key_a, nullptr, tb.idx_a, 0, 0);
+        full.run_if = nullptr;
+        checked = false;
+        sort_full(full, st, &L);
+    } else if (multi) {
+        const int shift = digit_shift64(pm, 0);
+        uint64_t *k0 = (pm & 1) ? tb.key_b : tb.key_a, *k0o = (pm & 1) ? tb.key_a : tb.key_b;
+        uint32_t *i0 = (pm & 1) ? tb.idx_b : tb.idx_a, *i0o = (pm & 1) ? tb.idx_a : tb.idx_b;
+        keys(k0, nullptr, i0, pm, shift);
+        passes(k0, k0o, i0, i0o, pm, shift, 0);  // result: idx_a
+        gather(tb.key3, tb.key_b, sys_id);
+        s1 = std::max(0, 63 - (8 * pm - tb.sys_bits));
+    } else if (p2 > 0) {
         uint64_t *k0 = (p2 & 1) ? tb.key_b : tb.key_a, *k0o = (p2 & 1) ? tb.key_a : tb.key_b;
         uint32_t *i0 = (p2 & 1) ? tb.idx_b : tb.idx_a, *i0o = (p2 & 1) ? tb.idx_a : tb.idx_b;
-        launch_pdl(k_keys, dim3(blocks_for(n, 256)), dim3(256), 0, st, tb.pos, n, tb.sc, tb.key3, k0, tb.key2, i0,
-                                                   multi ? tb.sys_id : nullptr, tb.sys_root, tb.single, 0);
-        L += 1;
-        cudaError_t e = sort_reset(tb.sort_scratch, n, st);
-        if (e == cudaSuccess)
-            e = sort_histograms(tb.key2, p2, 0, tb.key3, 8, 8, multi ? tb.sys_id : nullptr, 16, n, tb.sort_scratch,
-                                nullptr, st, &L);
-        if (e != cudaSuccess) return e;
-        passes(k0, k0o, i0, i0o, p2, p2, 0, nullptr, st);                   // result: key_a, idx_a
-        gather(tb.key3, tb.key_b, nullptr, st);                               // k1 in that order
-        passes(tb.key_b, tb.key_a, tb.idx_a, tb.idx_b, 8, 8, 8, nullptr, st);  // result: key_b, idx_a
+        keys(k0, tb.key2, i0, p2, digit_shift(p2, 0));
+        passes(k0, k0o, i0, i0o, p2, digit_shift(p2, 0), 0);              // result: key_a, idx_a
+        gather(tb.key3, tb.key_b, nullptr);                               // k1 in that order
+        passes(tb.key_b, tb.key_a, tb.idx_a, tb.idx_b, 8, 0, 8);          // result: key_b, idx_a
+        gather(tb.key2, tb.key_a, nullptr);                               // k2 in sorted order
+        checked = p2 < 8;
+        s2 = digit_shift(p2, 0);
     } else {
         uint64_t *k0 = (p1 & 1) ? tb.key_a : tb.key_b, *k0o = (p1 & 1) ? tb.key_b : tb.key_a;
         uint32_t *i0 = (p1 & 1) ? tb.idx_b : tb.idx_a, *i0o = (p1 & 1) ? tb.idx_a : tb.idx_b;
-        launch_pdl(k_keys, dim3(blocks_for(n, 256)), dim3(256), 0, st, tb.pos, n, tb.sc, tb.key3, k0, nullptr, i0, nullptr, tb.sys_root,
-                                                   tb.single, 1);
-        L += 1;
-        cudaError_t e = sort_reset(tb.sort_scratch, n, st);
-        if (e == cudaSuccess)
-            e = sort_histograms(tb.key3, p1, 8, nullptr, 0, 0, nullptr, 0, n, tb.sort_scratch, nullptr, st, &L);
-        if (e != cudaSuccess) return e;
-        passes(k0, k0o, i0, i0o, p1, p1, 8, nullptr, st);  // result: key_b, idx_a
+        keys(k0, nullptr, i0, p1, digit_shift(p1, 0));
+        passes(k0, k0o, i0, i0o, p1, digit_shift(p1, 0), 0);  // result: key_b, idx_a
+        s1 = digit_shift(p1, 0);
     }
     if (checked) {
         // Equal neighbours over the bits the plan sorted mean it did not separate
-        // every particle: short runs of them are sorted in place, and a long one
-        // makes the full sort run. Inside a stream capture the full sort is the
-        // body of a conditional graph node that runs only when the check sets its
-        // condition; launched directly, each of its kernels returns at once unless
-        // the flag is set.
-        if (p2 > 0) gather(tb.key2, tb.key_a, nullptr, st);  // k2 in sorted order, for the check and the runs
-        cudaGraphConditionalHandle cond = 0;
-        cudaGraph_t cg = nullptr;
-        cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-        const bool use_cond = tb.cond_stream && cudaStreamGetCaptureInfo(st, &cs, nullptr, &cg) == cudaSuccess &&
-                              cs == cudaStreamCaptureStatusActive &&
-                              cudaGraphConditionalHandleCreate(&cond, cg, 0, cudaGraphCondAssignDefault) == cudaSuccess;
-        if (!use_cond) cudaGetLastError();
+        // every particle: short runs of them are sorted in place (k2 is read, or
+        // computed, only where k1 is equal), and a long one makes the full sort run,
+        // a launch that otherwise returns at once.
         launch_pdl(k_fix_ties, dim3(blocks_for(n, 256)), dim3(256), 0, st, tb.key_b, tb.key_a, tb.idx_a, tb.pos,
-                   p2 > 0 ? 1 : 0, p2 > 0 ? 0 : digit_shift(p1, 0), p2 > 0 ? digit_shift(p2, 0) : 0, n, tb.single,
-                   tb.sc, cond, use_cond ? 1 : 0);
+                   p2 > 0 ? 1 : 0, s1, s2, n, tb.single, sys_sorted, tb.sys_root, tb.sc);
         L += 1;
-        cudaStream_t fs = st;
-        cudaError_t e;
-        if (use_cond) {
-            const cudaGraphNode_t *deps = nullptr;
-            size_t ndeps = 0;
-            if ((e = cudaStreamGetCaptureInfo(st, &cs, nullptr, &cg, &deps, &ndeps)) != cudaSuccess) return e;
-            cudaGraphNodeParams cp = {};
-            cp.type = cudaGraphNodeTypeConditional;
-            cp.conditional.handle = cond;
-            cp.conditional.type = cudaGraphCondTypeIf;
-            cp.conditional.size = 1;
-            cudaGraphNode_t node;
-            if ((e = cudaGraphAddNode(&node, cg, deps, ndeps, &cp)) != cudaSuccess) return e;
-            if ((e = cudaStreamUpdateCaptureDependencies(st, &node, 1, cudaStreamSetCaptureDependencies)) != cudaSuccess)
-                return e;
-            if ((e = cudaStreamBeginCaptureToGraph(tb.cond_stream, cp.conditional.phGraph_out[0], nullptr, nullptr, 0,
-                                                   cudaStreamCaptureModeRelaxed)) != cudaSuccess)
-                return e;
-            fs = tb.cond_stream;
-        }
-        // the full sort by (k1, k2): 8 passes on k2, the gather of k1, 8 passes on k1
-        const unsigned body_first = L;
-        if (p2 == 0) {
-            launch_pdl(k_keys_second, dim3(blocks_for(n, 256)), dim3(256), 0, fs, tb.pos, n, tb.sc, tb.key2, tb.single, ties);
-            L += 1;
-        }
-        if ((e = sort_histograms(tb.key2, 8, 18, tb.key3, 8, 26, nullptr, 0, n, tb.sort_scratch, ties, fs, &L)) !=
-            cudaSuccess)
-            return e;
-        launch_pdl(k_full_sort_init, dim3(blocks_for(n, 256)), dim3(256), 0, fs, tb.key2, tb.key_a, tb.idx_a, n, ties);
-        L += 1;
-        passes(tb.key_a, tb.key_b, tb.idx_a, tb.idx_b, 8, 8, 18, ties, fs);  // result: key_a, idx_a
-        gather(tb.key3, tb.key_b, ties, fs);
-        passes(tb.key_b, tb.key_a, tb.idx_a, tb.idx_b, 8, 8, 26, ties, fs);  // result: key_b, idx_a
-        gather(tb.key2, tb.key_a, ties, fs);                                  // k2 sorted
-        if (use_cond) {
-            cudaGraph_t body = nullptr;
-            if ((e = cudaStreamEndCapture(fs, &body)) != cudaSuccess) return e;
-            if (tb.cond_launches) *tb.cond_launches += L - body_first;
-        }
+        sort_full(full, st, &L);
     }
-    if (multi) {
-        // then by system (16-bit ids, 2 stable passes; result back in key_a / idx_a)
-        launch_pdl(k_gather_sys, dim3(blocks_for(n, 256)), dim3(256), 0, st, tb.sys_id, tb.idx_a, tb.key_a, nullptr, n);
-        passes(tb.key_a, tb.key_b, tb.idx_a, tb.idx_b, 2, 8, 16, nullptr, st);
-        gather(tb.key3, tb.key_b, nullptr, st);  // k1 sorted
-        launch_pdl(k_gather_sys, dim3(blocks_for(n, 256)), dim3(256), 0, st, tb.sys_id, tb.idx_a, nullptr, tb.sys_sorted, n);
-        L += 2;
-    }
-    // k2 sorted into key_a (a checked plan has it already, or needs none: with
-    // every k1 prefix distinct, nothing reads k2)
-    if (!checked) gather(tb.key2, tb.key_a, nullptr, st);
     if (tb.mass_ready && !multi) cudaStreamWaitEvent(st, tb.mass_ready, 0);  // the first reader of the masses
     launch_pdl(k_gather_bodies, dim3(blocks_for(n, 256)), dim3(256), 0, st, tb.idx_a, tb.pos, tb.mass, tb.body, n, tb.sc, tb.single);
     L += 1;
     *launches += L;
     if (n < 2) return cudaGetLastError();
     L = 0;
-    const uint32_t *sys_sorted = multi ? tb.sys_sorted : nullptr;
     launch_pdl(k_deep_groups, dim3(blocks_for(n, 256)), dim3(256), 0, st, tb.key_b, tb.key_a, tb.key3, tb.idx_a, tb.body, n,
                                                        sys_sorted, tb.sys_root, tb.sc, tb.single);
     KeyView kv{tb.key_b, tb.key_a, tb.key3, (int)n, sys_sorted};
     const uint32_t m = n - 1;
     launch_pdl(k_radix_tree, dim3(blocks_for(m, 256)), dim3(256), 0, st, kv, tb.bleft, tb.bright, tb.bparent, tb.leaf_bparent,
-                                                      tb.bdelta, &tb.sc->max_prefix_bits, tb.sc->pair_passes);
+                                                      tb.bdelta, &tb.sc->max_prefix_bits, tb.sc->pair_passes,
+               multi ? (uint32_t)tb.sys_bits : 0u);
     launch_pdl(k_head_flags, dim3(blocks_for(n, 256)), dim3(256), 0, st, tb.bparent, tb.bdelta, m, tb.head_flag,
                tb.head_id, tb.oparent, tb.leaf_oparent, tb.ocount);
     L += 3 + scan_exclusive(tb.head_id, m, tb.scan_tmp, &tb.sc->n_onodes, st);

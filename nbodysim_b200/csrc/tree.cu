@@ -723,6 +723,9 @@ __global__ void k_collapse(const int32_t *__restrict__ bleft, const int32_t *__r
 // as the reference computes them. A child separated from its parent by k
 // single-child chain nodes enters with its centre of mass passed k times
 // through the chain's (c * m) / m, the value the reference's chain top holds.
+constexpr int kComLanes = 4;
+constexpr uint32_t kComGroupsMax = 131072;
+
 __device__ inline double3 load_node_com(const double4 *p, double &m) {
     const double2 *q = reinterpret_cast<const double2 *>(p);
     double2 a = __ldcg(q), b = __ldcg(q + 1);
@@ -787,8 +790,7 @@ __device__ inline double4 node_com(const double4 *__restrict__ body, int4 c0, in
 template <typename T>
 // (launch bounds: 4 resident blocks of 256 threads, 64 registers)
 __global__ void __launch_bounds__(256, 4)
-    k_com(const double4 *__restrict__ body, const int32_t *__restrict__ leaf_oparent,
-          const int32_t *__restrict__ oparent, const int32_t *__restrict__ ochild,
+    k_com(const double4 *__restrict__ body, const int32_t *__restrict__ oparent, const int32_t *__restrict__ ochild,
           const int32_t *__restrict__ ometa, double4 *onode, uint32_t *ocount, uint32_t n, DevScalars *sc) {
     griddep();
     // One thread per node; the climb starts at nodes whose children are all
@@ -828,6 +830,123 @@ __global__ void __launch_bounds__(256, 4)
         __stcg(q, make_double2(out.x, out.y));
         __stcg(q + 1, make_double2(out.z, out.w));
         p = up;
+    }
+}
+
+// A node is computed by kComLanes lanes: each loads the children k = lane, lane +
+// kComLanes, ... at once, passes them through their chains and forms the products;
+// the sums then run over the children in order, every lane taking each term by
+// shuffle, and the three quotients are taken by three lanes.
+//
+// Bound: latency of a hop (count, structure, children), of which a climb has as many
+// as the octree has levels. One thread per node (k_com) loads the children one after
+// another, up to 8 round trips to L2 a hop; with many nodes, whose hops overlap, its
+// fewer instructions win. This against k_com: 1000 particles 16 / 29 us, 5000 18 / 39,
+// 65,536 25 / 43, 100,000 33 / 47, 200,000 63 / 54, 1,048,576 231 / 154 (2 lanes: 20,
+// 25, -, 33, 63, 223; 8 lanes: 16, 16, -, 33, 74, 293).
+template <typename T>
+__device__ inline T group_value(T v, int k) { return __shfl_sync(0xffffffffu, v, k, kComLanes); }
+
+template <typename T>
+__global__ void __launch_bounds__(256)
+    k_com_groups(const double4 *__restrict__ body, const int32_t *__restrict__ oparent,
+                 const int32_t *__restrict__ ochild, const int32_t *__restrict__ ometa, double4 *onode, uint32_t *ocount,
+                 uint32_t n, DevScalars *sc) {
+    griddep();
+    constexpr int kEach = 8 / kComLanes;  // children per lane
+    const unsigned FULL = 0xffffffffu;
+    // The climb starts at nodes whose children are all bodies; a node is computed
+    // by the group of its last node child to finish.
+    const uint32_t q = (blockIdx.x * blockDim.x + threadIdx.x) / kComLanes;
+    const int l = threadIdx.x % kComLanes;
+    int p = -1;
+    if (q < n - 1 && q < sc->n_onodes && meta_ninternal(ometa[q]) == 0) p = (int)q;
+    // A well-formed tree is at most kMaxLevels + 1 internal levels deep; the
+    // bound only guards against a malformed tree after a reported error.
+    for (int hops = 0; __any_sync(FULL, p >= 0); hops++) {
+        if (hops > kMaxLevels + 1 || p >= (int)(n - 1)) {
+            atomicOr(&sc->status, kStatusCapacity);
+            p = -1;
+            if (hops > kMaxLevels + 1) return;  // (the same hop for the whole warp)
+        }
+        // The node's structure is final (the collapse wrote it): it loads before the
+        // arrival count, so that after it only the children's values remain to be read.
+        int meta = 0, up = -1;
+        int32_t ch[kEach];
+        if (p >= 0) {
+            meta = ometa[p];
+            up = oparent[p];
+#pragma unroll
+            for (int i = 0; i < kEach; i++) ch[i] = __ldg(&ochild[8 * (size_t)p + l + i * kComLanes]);
+        }
+        const int nch = meta_nchild(meta), L = meta_level(meta);
+        if (hops > 0) {
+            // One acquire-release count per node: it publishes the node this group wrote
+            // on the previous hop, and the last node child to arrive sees every other
+            // child's result. (The only node child needs none.)
+            __syncwarp();
+            uint32_t old = 0;
+            if (p >= 0 && l == 0 && meta_ninternal(meta) > 1)
+                asm volatile("atom.acq_rel.gpu.global.add.u32 %0, [%1], 1;" : "=r"(old) : "l"(&ocount[p]) : "memory");
+            old = group_value(old, 0);
+            __syncwarp();
+            if (old != (uint32_t)(meta_ninternal(meta) - 1)) p = -1;
+        }
+        T cm[kEach], px[kEach], py[kEach], pz[kEach];
+#pragma unroll
+        for (int i = 0; i < kEach; i++) {
+            cm[i] = px[i] = py[i] = pz[i] = T(0);
+            if (p < 0 || l + i * kComLanes >= nch) continue;
+            const int c = ch[i];
+            T cmk, cx, cy, cz;
+            int chain = 0;
+            if (c < 0) {
+                const double4 b = body[~c];
+                cmk = (T)b.w;
+                cx = (T)b.x; cy = (T)b.y; cz = (T)b.z;
+            } else {
+                double dm;
+                const double3 cc = load_node_com(&onode[c], dm);
+                cmk = (T)dm;
+                cx = (T)cc.x; cy = (T)cc.y; cz = (T)cc.z;
+                chain = meta_level(ometa[c]) - L - 1;
+            }
+            for (int t = 0; t < chain; t++) {
+                if (cmk == T(0)) {
+                    cx = cy = cz = T(0);
+                } else {
+                    cx = div_rn(mul_rn(cx, cmk), cmk);
+                    cy = div_rn(mul_rn(cy, cmk), cmk);
+                    cz = div_rn(mul_rn(cz, cmk), cmk);
+                }
+            }
+            cm[i] = cmk;
+            px[i] = mul_rn(cx, cmk); py[i] = mul_rn(cy, cmk); pz[i] = mul_rn(cz, cmk);
+        }
+        // The reference sums the masses, then the mass-weighted centres, each in
+        // child order; the terms past the last child are +0 and change nothing.
+        T m = 0, sx = 0, sy = 0, sz = 0;
+        const int most = (int)__reduce_max_sync(FULL, p >= 0 ? (unsigned)nch : 0u);
+#pragma unroll
+        for (int i = 0; i < kEach; i++) {
+            if (i * kComLanes >= most) break;
+#pragma unroll
+            for (int k = 0; k < kComLanes; k++) {
+                m = add_rn(m, group_value(cm[i], k));
+                sx = add_rn(sx, group_value(px[i], k));
+                sy = add_rn(sy, group_value(py[i], k));
+                sz = add_rn(sz, group_value(pz[i], k));
+            }
+        }
+        if (p >= 0) {
+            double *out = reinterpret_cast<double *>(&onode[p]);
+#pragma unroll
+            for (int d = l; d < 4; d += kComLanes) {
+                const T num = d == 0 ? sx : d == 1 ? sy : sz;
+                __stcg(out + d, d == 3 ? (double)m : m == T(0) ? 0.0 : (double)div_rn(num, m));
+            }
+        }
+        p = p >= 0 ? up : -1;
     }
 }
 
@@ -955,12 +1074,10 @@ cudaError_t compute_com(const TreeBuild &tb, cudaStream_t st, unsigned *launches
     const uint32_t n = tb.n;
     if (n < 2) return cudaSuccess;
     // (the arrival counts were zeroed by the build's k_head_flags)
-    if (tb.single)
-        launch_pdl(k_com<float>, dim3(blocks_for(n - 1, 256)), dim3(256), 0, st, tb.body, tb.leaf_oparent, tb.oparent, tb.ochild,
-                                                             tb.ometa, tb.onode, tb.ocount, n, tb.sc);
-    else
-        launch_pdl(k_com<double>, dim3(blocks_for(n - 1, 256)), dim3(256), 0, st, tb.body, tb.leaf_oparent, tb.oparent, tb.ochild,
-                                                              tb.ometa, tb.onode, tb.ocount, n, tb.sc);
+    const bool groups = n <= kComGroupsMax;
+    const dim3 grid(blocks_for((uint64_t)(n - 1) * (groups ? kComLanes : 1), 256));
+    launch_pdl(groups ? (tb.single ? k_com_groups<float> : k_com_groups<double>) : tb.single ? k_com<float> : k_com<double>,
+               grid, dim3(256), 0, st, tb.body, tb.oparent, tb.ochild, tb.ometa, tb.onode, tb.ocount, n, tb.sc);
     *launches += 1;
     return cudaGetLastError();
 }

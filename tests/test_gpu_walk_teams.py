@@ -38,8 +38,10 @@ def test_team_equals_single_warp_with_a_long_queue(nb, precision):
         assert np.array_equal(e.get_particles(acc=True)[2][:3000], own)
 
 
-@pytest.mark.parametrize("precision,n", [(0, 56832), (0, 56833), (1, 113664), (1, 113665)])
-def test_counts_on_both_sides_of_the_team_limit(nb, orc, precision, n):
+@pytest.mark.parametrize("precision,n", [(0, 56832), (0, 56833), (1, 113664), (1, 113665), (1, 131072), (1, 131073)])
+def test_counts_on_both_sides_of_the_size_limits(nb, orc, precision, n):
+    """Teams end at 56,832 (MIXED) and 113,664 (FP64) particles, the mass pass's groups
+    of lanes per node at 131,072."""
     pos, vel, mass = nb.generate(n, gen_type=2, size=1024.0, seed=n)
     sample = np.sort(np.random.default_rng(n).choice(n, 300, replace=False)).astype(np.uint32)
     sample[-1] = n - 1

@@ -14,6 +14,7 @@
 // its loads and used 44% of the pipe; with few targets most of the chip was idle.
 // 100,000 particles: 3.40 -> 1.33 ms for 4096 targets, 2.05 -> 0.12 ms for 100.
 #include "direct.cuh"
+#include "fp64.cuh"
 
 namespace nbody {
 
@@ -44,23 +45,6 @@ constexpr uint32_t kDirectSlab = 65536;   // targets per launch: bounds the chun
 __device__ inline double pair_factor(double r2, double gm, bool damping) {
     const double r = __dsqrt_rn(r2);
     return __ddiv_rn(__ddiv_rn(gm, damping ? r2 + exp(-r) : r2), r);
-}
-
-// Whether r^-3 stays well inside the exponent range (false for zero, subnormal, NaN).
-__device__ inline bool plain_range(double r2) { return (uint32_t)(__double2hiint(r2) >> 20) - 400u < 1250u; }
-
-// G M r^-3 within plain_range: the hardware's approximate r^-1 (y), corrected in the
-// cube by the binomial series of (1 - e)^(-3/2) = 1 + 3/2 e + 15/8 e^2 + ..., where
-// e = 1 - r^2 y^2 includes what the rounding of r^2 y left; e < 2^-20, so the next
-// term is below 2^-58. Root mean square error of a single pair's force against an
-// 80-bit one: 1.52e-16 (with a square root and divides it was 1.57e-16).
-__device__ inline double pair_factor_plain(double r2, double gm) {
-    double y;
-    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(r2));
-    const double h = __dmul_rn(r2, y);
-    const double e = fma(-fma(r2, y, -h), y, fma(-h, y, 1.0));
-    const double p = __dmul_rn(gm, __dmul_rn(__dmul_rn(y, y), y));
-    return fma(p, __dmul_rn(e, fma(e, 1.875, 1.5)), p);
 }
 
 __device__ inline void combine_lanes(double &s, double &c, int lane) {
@@ -112,7 +96,7 @@ double f[kTargets], dx[kTargets], dy[kTargets], dz[kTargets], r2[kTargets];
             dx[q] = __dsub_rn(x, xi[q]); dy[q] = __dsub_rn(y, yi[q]); dz[q] = __dsub_rn(z, zi[q]);
             r2[q] = __dadd_rn(__dadd_rn(__dmul_rn(dx[q], dx[q]), __dmul_rn(dy[q], dy[q])), __dmul_rn(dz[q], dz[q]));
             if constexpr (!kDamp) {
-                f[q] = pair_factor_plain(r2[q], gm);
+                f[q] = inverse_cube(r2[q], gm);
                 rare |= !plain_range(r2[q]);
             }
         }

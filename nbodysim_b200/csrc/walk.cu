@@ -30,6 +30,7 @@
 // FP64 ("plain form"): the same walk with every quantity in FP64 and the
 // reference's opening test evaluated directly.
 #include "walk.cuh"
+#include "fp64.cuh"
 
 #include <type_traits>
 
@@ -79,7 +80,8 @@ struct TileSmem<false> {
 template <>
 struct TileSmem<true> {
     alignas(16) double4 tc[32];  // com.xyz (absolute), side
-    int2 tr[32];                 // reach mask, node ref
+    double tq[32];               // (side/theta)^2
+    uint32_t tr[32];             // reach mask
 };
 
 // Shared memory of one group: its interaction lists, rings of kCap entries that
@@ -319,7 +321,7 @@ __device__ inline void pair_adjoint(T dx, T dy, T dz, T r2, T gm, T lax, T lay, 
         vz = gm * (g * laz + c * uz);
         mterm = float(kG) * gr * sh;
     } else {
-        const T inv = 1.0 / sqrt(r2);
+        const T inv = plain_range(r2) ? inverse_root(r2) : 1.0 / sqrt(r2);
         const T inv2 = inv * inv;
         T g, h;
         if constexpr (kDamp) {
@@ -449,23 +451,33 @@ __device__ inline void adj_list_f64(const double4 *lc, const uint32_t *lm, const
     }
 }
 
+// FP64 pair terms. Bound: the FP64 pipe and its dependent chains. A square root and a
+// divide per pair (and per opening test of a mixed node) were most of the walk; the
+// corrected inverse roots (fp64.cuh) and the test on squares take 16,384 particles from
+// 227 to 147 us, 200,000 from 1750 to 1107, 60,001 damped (which keeps a divide and an
+// exponential) from 890 to 790, the adjoint of 16,384 from 302 to 255.
 template <bool kDamp, bool kPot>
 __device__ inline void force_list_f64(const double4 *lc, const uint32_t *lm, int count, int lane, double bx,
                                       double by, double bz, double &ax, double &ay, double &az, double &pot) {
 #pragma unroll 2
     for (int k = 0; k < count; k++) {
-        const uint32_t m = lm[k];
-        if (!((m >> lane) & 1u)) continue;
+        const bool take = (lm[k] >> lane) & 1u;
         const double4 c = lc[k];
         const double dx = c.x - bx, dy = c.y - by, dz = c.z - bz;
         const double r2 = dx * dx + dy * dy + dz * dz;
-        const double d = sqrt(r2);
-        const double inv = 1.0 / d;
-        double f;
-        if constexpr (kDamp) f = c.w * inv / (r2 + exp(-d));
-        else f = c.w * inv * inv * inv;
+        double f, inv = 0.0;
+        if constexpr (kDamp || kPot) inv = inverse_root(r2);
+        if constexpr (kDamp) f = c.w * inv / (r2 + exp(-(r2 * inv)));
+        else f = inverse_cube(r2, c.w);
+        if (!plain_range(r2)) {  // the lane's own leaf (not taken), or an extreme distance
+            const double d = sqrt(r2);
+            inv = 1.0 / d;
+            if constexpr (kDamp) f = c.w * inv / (r2 + exp(-d));
+            else f = c.w * inv * inv * inv;
+        }
+        f = take ? f : 0.0;
         ax = fma(f, dx, ax); ay = fma(f, dy, ay); az = fma(f, dz, az);
-        if constexpr (kPot) pot += c.w * inv;
+        if constexpr (kPot) pot += take ? c.w * inv : 0.0;
     }
 }
 
@@ -738,11 +750,12 @@ __global__ void __launch_bounds__((kTeam ? kTeamMaxWarps : kWalkMaxWarps) * 32) 
             uint32_t my_open = 0;
             bool mixed = false;
             float r2box = 0.f;  // squared distance of the node from the group's box (MIXED form)
+            double qd = 0.0;             // (side/theta)^2 (FP64 form)
             float qf = 0.f, band = 0.f;  // (side/theta)^2 in FP32 and the half-width of its error band
             if (is_int) {
                 if constexpr (kFp64) {
                     const double sq = s.gc.S * so / theta;
-                    const double qd = sq * sq;
+                    qd = sq * sq;
                     const double ox = cx - s.gc.ref[0], oy = cy - s.gc.ref[1], oz = cz - s.gc.ref[2];
                     const double ax_ = fmax(fmax(dlox - ox, ox - dhix), 0.0), ay_ = fmax(fmax(dloy - oy, oy - dhiy), 0.0),
                                  az_ = fmax(fmax(dloz - oz, oz - dhiz), 0.0);
@@ -779,18 +792,26 @@ __global__ void __launch_bounds__((kTeam ? kTeamMaxWarps : kWalkMaxWarps) * 32) 
             if (intm) {
                 if constexpr (kFp64) {
                     tile.tc[lane] = make_double4(cx, cy, cz, s.gc.S * so);
-                    tile.tr[lane] = make_int2((int)reach, ref);
+                    tile.tq[lane] = qd;
+                    tile.tr[lane] = reach;
                     __syncwarp();
                 }
                 if constexpr (kFp64) {
-                    // the FP64 form decides every mixed node with the reference's own test
+                    // The FP64 form compares squares, which settles all but distances within
+                    // their rounding (the FLOAT build's: grp_rel) of the opening radius; those
+                    // take the reference's own test, a square root and a divide.
                     uint32_t mm = intm;
                     while (mm) {
                         const int k = __ffs(mm) - 1;
                         mm &= mm - 1;
                         const double4 c = tile.tc[k];
-                        const uint32_t rk = (uint32_t)tile.tr[k].x;
-                        const bool open = ref_open(single, c.x, c.y, c.z, b.x, b.y, b.z, c.w, theta, theta_f);
+                        const double q_k = tile.tq[k];
+                        const uint32_t rk = tile.tr[k];
+                        const double dx = c.x - b.x, dy = c.y - b.y, dz = c.z - b.z;
+                        const double over = dx * dx + dy * dy + dz * dz - q_k;
+                        bool open = over < 0.0;
+                        if (!(fabs(over) > grp_rel * q_k))
+                            open = ref_open(single, c.x, c.y, c.z, b.x, b.y, b.z, c.w, theta, theta_f);
                         const uint32_t om = __ballot_sync(FULL, open) & rk;
                         if (lane == k) my_open = om;
                     }

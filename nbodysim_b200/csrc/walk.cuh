@@ -25,8 +25,9 @@ constexpr int kTeamList = 32 + 32 * kTeamMaxWarps;
 // cost more than the last wave of single warps. Walk times, team against single
 // warps (us): MIXED 5000 particles 51 / 103, shell of 20,011 50 / 89, cubes of 48,000
 // 170 / 197, 56,000 195 / 206 and 70,000 240 / 228; its adjoint 5000 89 / 183, 85,000
-// 578 / 598, 100,000 682 / 648; FP64 5000 135 / 375, 16,384 226 / 580, 60,001 885 /
-// 1168, 112,000 1006 / 1235; its adjoint 16,384 310 / 671, 100,000 1460 / 1591.
+// 578 / 598, 100,000 682 / 648; FP64 (with the pair terms of then) 5000 135 / 375,
+// 16,384 226 / 580, 60,001 885 / 1168, 112,000 1006 / 1235; its adjoint 16,384 310 /
+// 671, 100,000 1460 / 1591.
 // Systems of fewer than kTeamMinSize particles have a few short tiles per group, for
 // which the barriers cost more (a step of 97: 133 us with teams, 125 without; 150:
 // the same; 300: 147 and 151).

@@ -176,8 +176,9 @@ typedef struct nbody_stats {
     uint64_t merged_collisions; /* particles removed by collision merges in the last nbody_step */
     uint64_t collision_pairs;  /* (particle, leaf) pairs found within range, last nbody_step */
     uint32_t sort_passes;      /* 8-bit radix-sort passes of the last tree build: the planned ones,
-                                  plus the full sort's 16 when the plan left a run of more than
-                                  64 equal neighbours */
+                                  plus the full sort's 16 (several systems: 18) when the plan left
+                                  a run of more than 64 equal neighbours; 0 for a system of at most
+                                  1024 particles, which is built without a sort plan */
     uint32_t sort_split_bits;  /* key bits (3 per octree level) that separate every pair of
                                   Morton neighbours in the last build */
     uint32_t sort_tie_runs;    /* runs of neighbours equal over the planned bits (at most 64 each)

@@ -347,7 +347,9 @@ int check_status(nbody_ctx *c) {
     s.root_side = h.root_side;
     s.sort_split_bits = h.max_prefix_bits;
     s.sort_tie_runs = h.tie_runs;
-    if (c->tb.nsys > 1) {
+    if (is_small_tree(c->tb)) {
+        s.sort_passes = 0;  // sorted within one block; the plans stay
+    } else if (c->tb.nsys > 1) {
         const int used = c->multi_step_call ? c->sort_deep_pm : c->sort_pm;
         s.sort_passes = used == 0 ? 18u : (uint32_t)used + (h.word_ties ? 18u : 0u);
         next_systems_plan(c, h);

@@ -431,12 +431,10 @@ __global__ void k_gather_bodies(const uint32_t *__restrict__ idx, const double *
 // levels mean coincident particles (the reference recurses without bound).
 constexpr int kMaxDeepGroup = 64;
 
-__global__ void k_deep_groups(const uint64_t *__restrict__ key1, const uint64_t *__restrict__ key2,
-                              uint64_t *__restrict__ key3, uint32_t *__restrict__ idx,
-                              double4 *__restrict__ body, uint32_t n, const uint32_t *__restrict__ sys,
-                              const double *__restrict__ sys_root, DevScalars *sc, int single) {
-    griddep();
-    uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+// Position i: the first of such a group handles it. `root`: center, side (one system).
+__device__ inline void deep_group_at(uint32_t i, const uint64_t *key1, const uint64_t *key2, uint64_t *key3,
+                                     uint32_t *idx, double4 *body, uint32_t n, const uint32_t *sys,
+                                     const double *sys_root, const double *one_root, DevScalars *sc, int single) {
     if (i + 1 >= n) return;
     const uint64_t k = key1[i], kk = key2[i];
     const uint32_t ss = sys ? sys[i] : 0u;
@@ -456,11 +454,8 @@ __global__ void k_deep_groups(const uint64_t *__restrict__ key1, const uint64_t 
         atomicOr(&sc->status, kStatusCoincident);
         return;
     }
-    double root[4] = {sc->root_center[0], sc->root_center[1], sc->root_center[2], sc->root_side};
-    if (sys) {
-        const double *r = sys_root + 4 * (size_t)ss;
-        root[0] = r[0]; root[1] = r[1]; root[2] = r[2]; root[3] = r[3];
-    }
+    const double *r = sys ? sys_root + 4 * (size_t)ss : one_root;
+    const double root[4] = {r[0], r[1], r[2], r[3]};
     for (uint32_t j = i; j <= e; j++) {
         const double4 b = body[j];
         const double p[3] = {b.x, b.y, b.z};
@@ -483,6 +478,15 @@ __global__ void k_deep_groups(const uint64_t *__restrict__ key1, const uint64_t 
     }
     for (uint32_t j = i; j < e; j++)
         if (key3[j] == key3[j + 1]) atomicOr(&sc->status, kStatusCoincident);
+}
+
+__global__ void k_deep_groups(const uint64_t *__restrict__ key1, const uint64_t *__restrict__ key2,
+                              uint64_t *__restrict__ key3, uint32_t *__restrict__ idx,
+                              double4 *__restrict__ body, uint32_t n, const uint32_t *__restrict__ sys,
+                              const double *__restrict__ sys_root, DevScalars *sc, int single) {
+    griddep();
+    const double root[4] = {sc->root_center[0], sc->root_center[1], sc->root_center[2], sc->root_side};
+    deep_group_at(blockIdx.x * blockDim.x + threadIdx.x, key1, key2, key3, idx, body, n, sys, sys_root, root, sc, single);
 }
 
 // ---------------------------------------------------------------------------
@@ -527,6 +531,32 @@ struct DeltaFrom {
     }
 };
 
+// Binary node i, whose first pair of neighbours shares dn bits: its children, encoded
+// >= 0 internal binary node, < 0 leaf ~index. Returns its prefix length.
+__device__ inline int radix_node(const KeyView &kv, int i, int dn, int &left, int &right) {
+    const DeltaFrom di(kv, i);
+    const int dprev = di(i - 1);
+    int d = (dn - dprev) >= 0 ? 1 : -1;
+    int dmin = d > 0 ? dprev : dn;  // delta(i, i - d)
+    int lmax = 2;
+    while (di(i + lmax * d) > dmin) lmax <<= 1;
+    int l = 0;
+    for (int t = lmax >> 1; t >= 1; t >>= 1)
+        if (di(i + (l + t) * d) > dmin) l += t;
+    int j = i + l * d;
+    int dnode = di(j);
+    int s = 0, t = l;
+    do {
+        t = (t + 1) >> 1;
+        if (di(i + (s + t) * d) > dnode) s += t;
+    } while (t > 1);
+    int gamma = i + s * d + min(d, 0);
+    int lo = min(i, j), hi = max(i, j);
+    left = (lo == gamma) ? ~gamma : gamma;
+    right = (hi == gamma + 1) ? ~(gamma + 1) : gamma + 1;
+    return dnode;
+}
+
 __global__ void k_radix_tree(KeyView kv, int32_t *__restrict__ bleft, int32_t *__restrict__ bright,
                              int32_t *__restrict__ bparent, int32_t *__restrict__ leaf_bparent,
                              int32_t *__restrict__ bdelta, uint32_t *max_prefix_bits, uint32_t *pair_passes,
@@ -559,27 +589,8 @@ __global__ void k_radix_tree(KeyView kv, int32_t *__restrict__ bleft, int32_t *_
         return;
     }
     const bool seg_root = i == 0 || (kv.sys && kv.sys[i - 1] != kv.sys[i]);
-    const DeltaFrom di(kv, i);
-    const int dprev = di(i - 1);
-    int d = (dn - dprev) >= 0 ? 1 : -1;
-    int dmin = d > 0 ? dprev : dn;  // delta(i, i - d)
-    int lmax = 2;
-    while (di(i + lmax * d) > dmin) lmax <<= 1;
-    int l = 0;
-    for (int t = lmax >> 1; t >= 1; t >>= 1)
-        if (di(i + (l + t) * d) > dmin) l += t;
-    int j = i + l * d;
-    int dnode = di(j);
-    int s = 0, t = l;
-    do {
-        t = (t + 1) >> 1;
-        if (di(i + (s + t) * d) > dnode) s += t;
-    } while (t > 1);
-    int gamma = i + s * d + min(d, 0);
-    int lo = min(i, j), hi = max(i, j);
-    // children encoded: >= 0 internal binary node, < 0 leaf ~index
-    int left = (lo == gamma) ? ~gamma : gamma;
-    int right = (hi == gamma + 1) ? ~(gamma + 1) : gamma + 1;
+    int left, right;
+    const int dnode = radix_node(kv, i, dn, left, right);
     bleft[i] = left;
     bright[i] = right;
     bdelta[i] = dnode;
@@ -625,6 +636,62 @@ __global__ void k_sys_roots(const uint32_t *__restrict__ sys_start, const uint32
     root_node[s] = (b - a >= 2 && flag[a]) ? (int32_t)head_id[a] : -1;
 }
 
+// Visits, left to right, the exits of the same-level (L) binary subtree of head i.
+template <class Emit>
+__device__ inline void collapse_node(int i, int L, const int32_t *bleft, const int32_t *bright, const int32_t *bdelta,
+                                     Emit &&emit, uint32_t *status) {
+    auto same_level = [&](int ch) { return ch >= 0 && level_of(bdelta[ch]) == L; };
+    if (L >= kMaxLevels) {
+        // The capped level (keys equal over every word: coincident particles,
+        // reported as such) can nest deeper: an in-order walk with a stack, a
+        // frame visiting its left child, then its right child.
+        int fnode[8], fstate[8];
+        int fs = 1;
+        fnode[0] = i;
+        fstate[0] = 0;
+        while (fs > 0) {
+            const int x = fnode[fs - 1];
+            if (fstate[fs - 1] == 2) { fs--; continue; }
+            const int ch = fstate[fs - 1] == 0 ? bleft[x] : bright[x];
+            fstate[fs - 1]++;
+            if (same_level(ch)) {
+                if (fs < 8) { fnode[fs] = ch; fstate[fs] = 0; fs++; }
+                else atomicOr(status, kStatusCapacity);
+            } else {
+                emit(ch);
+            }
+        }
+    } else {
+        // In-order walk over the same-level binary nodes. Their prefix lengths grow
+        // strictly downwards and stay within the level's 3 key bits, so the walk is
+        // at most 3 binary nodes deep: unrolled, with nothing in local memory.
+        const int c1[2] = {bleft[i], bright[i]};
+    #pragma unroll
+        for (int a = 0; a < 2; a++) {
+            const int x = c1[a];
+            if (!same_level(x)) {
+                emit(x);
+                continue;
+            }
+            const int c2[2] = {bleft[x], bright[x]};
+    #pragma unroll
+            for (int b = 0; b < 2; b++) {
+                const int y = c2[b];
+                if (!same_level(y)) {
+                    emit(y);
+                    continue;
+                }
+                const int c3[2] = {bleft[y], bright[y]};
+    #pragma unroll
+                for (int c = 0; c < 2; c++) {
+                    if (same_level(c3[c])) atomicOr(status, kStatusCapacity);  // deeper than 3: malformed
+                    else emit(c3[c]);
+                }
+            }
+        }
+    }
+}
+
 // Each head gathers, left to right, the exits of its same-level binary
 // subtree: leaves and deeper heads. Left-to-right is Morton order, i.e. the
 // reference's child order 0..7.
@@ -657,56 +724,7 @@ __global__ void k_collapse(const int32_t *__restrict__ bleft, const int32_t *__r
         }
         nch++;
     };
-    auto same_level = [&](int ch) { return ch >= 0 && level_of(bdelta[ch]) == L; };
-    if (L >= kMaxLevels) {
-        // The capped level (keys equal over every word: coincident particles,
-        // reported as such) can nest deeper: an in-order walk with a stack, a
-        // frame visiting its left child, then its right child.
-        int fnode[8], fstate[8];
-        int fs = 1;
-        fnode[0] = (int)i;
-        fstate[0] = 0;
-        while (fs > 0) {
-            const int x = fnode[fs - 1];
-            if (fstate[fs - 1] == 2) { fs--; continue; }
-            const int ch = fstate[fs - 1] == 0 ? bleft[x] : bright[x];
-            fstate[fs - 1]++;
-            if (same_level(ch)) {
-                if (fs < 8) { fnode[fs] = ch; fstate[fs] = 0; fs++; }
-                else atomicOr(&sc->status, kStatusCapacity);
-            } else {
-                emit(ch);
-            }
-        }
-    } else {
-        // In-order walk over the same-level binary nodes. Their prefix lengths grow
-        // strictly downwards and stay within the level's 3 key bits, so the walk is
-        // at most 3 binary nodes deep: unrolled, with nothing in local memory.
-        const int c1[2] = {bleft[i], bright[i]};
-    #pragma unroll
-        for (int a = 0; a < 2; a++) {
-            const int x = c1[a];
-            if (!same_level(x)) {
-                emit(x);
-                continue;
-            }
-            const int c2[2] = {bleft[x], bright[x]};
-    #pragma unroll
-            for (int b = 0; b < 2; b++) {
-                const int y = c2[b];
-                if (!same_level(y)) {
-                    emit(y);
-                    continue;
-                }
-                const int c3[2] = {bleft[y], bright[y]};
-    #pragma unroll
-                for (int c = 0; c < 2; c++) {
-                    if (same_level(c3[c])) atomicOr(&sc->status, kStatusCapacity);  // deeper than 3: malformed
-                    else emit(c3[c]);
-                }
-            }
-        }
-    }
+    collapse_node((int)i, L, bleft, bright, bdelta, emit, &sc->status);
     ometa[id] = L | (min(nch, 8) << 8) | (min(nint, 8) << 12);
     if (id == 0) oparent[0] = -1;
     // the deepest level: one atomic per group of converged lanes
@@ -740,26 +758,25 @@ __device__ inline double div_rn(double a, double b) { return __ddiv_rn(a, b); }
 __device__ inline float div_rn(float a, float b) { return __fdiv_rn(a, b); }
 
 // One node's mass and centre of mass from its children, in the arithmetic of
-// T (double, or float for the reference's FLOAT build).
-// The node's child list comes in as c0, c1 (its eight slots).
-template <typename T>
-__device__ inline double4 node_com(const double4 *__restrict__ body, int4 c0, int4 c1,
-                                   const int32_t *__restrict__ ometa, const double4 *onode, int L, int nch) {
+// T (double, or float for the reference's FLOAT build): child(k) is the k-th child,
+// body_at(j) a body, node_at(c, mass, level) a node child's centre, mass and level.
+template <typename T, class Child, class BodyAt, class NodeAt>
+__device__ inline double4 node_com(int L, int nch, Child &&child, BodyAt &&body_at, NodeAt &&node_at) {
     T m = 0, sx = 0, sy = 0, sz = 0;
     for (int k = 0; k < nch; k++) {
-        const int4 h = k < 4 ? c0 : c1;  // selects, not an indexed array (which would live in local memory)
-        const int c = (k & 2) ? ((k & 1) ? h.w : h.z) : ((k & 1) ? h.y : h.x);
+        const int c = child(k);
         T cmk, cx, cy, cz;
         if (c < 0) {
-            const double4 b = body[~c];
+            const double4 b = body_at(~c);
             cmk = (T)b.w;
             cx = (T)b.x; cy = (T)b.y; cz = (T)b.z;
         } else {
             double dm;
-            const double3 cc = load_node_com(&onode[c], dm);
+            int level;
+            const double3 cc = node_at(c, dm, level);
             cmk = (T)dm;
             cx = (T)cc.x; cy = (T)cc.y; cz = (T)cc.z;
-            const int chain = meta_level(ometa[c]) - L - 1;
+            const int chain = level - L - 1;
             for (int t = 0; t < chain; t++) {
                 if (cmk == T(0)) {
                     cx = cy = cz = T(0);
@@ -825,7 +842,18 @@ __global__ void __launch_bounds__(256, 4)
         // The reference sums the masses, then the mass-weighted centres, each in
         // child order; both sums run here in one pass over the children.
         const int L = meta_level(meta);
-        const double4 out = node_com<T>(body, c0, c1, ometa, onode, L, nch);
+        const double4 out = node_com<T>(
+            L, nch,
+            [&](int k) {  // selects, not an indexed array (which would live in local memory)
+                const int4 h = k < 4 ? c0 : c1;
+                return (k & 2) ? ((k & 1) ? h.w : h.z) : ((k & 1) ? h.y : h.x);
+            },
+            [&](int j) { return body[j]; },
+            [&](int c, double &m, int &level) {
+                const double3 v = load_node_com(&onode[c], m);
+                level = meta_level(ometa[c]);
+                return v;
+            });
         double2 *q = reinterpret_cast<double2 *>(&onode[p]);
         __stcg(q, make_double2(out.x, out.y));
         __stcg(q + 1, make_double2(out.z, out.w));
@@ -951,6 +979,260 @@ __global__ void __launch_bounds__(256)
 }
 
 // ---------------------------------------------------------------------------
+// The whole build of a small system (root cube to mass and centre of mass) in one
+// block, with keys, trees and node values in shared memory: one thread per particle,
+// per binary node and per octree node.
+//
+// Bound of the general chain at these sizes: the latency of a dozen dependent
+// kernels (3 to 6 us each, whatever they do). A step of 97 particles takes 84 us
+// against 107 with the chain, of 600 109 against 134, of 1000 121 against 137. One thread per particle keeps every phase one pass; 1024 is the
+// largest block.
+struct SmallTree {
+    uint64_t k1[kSmallTree], k2[kSmallTree], k3[kSmallTree];
+    double4 body[kSmallTree], node[kSmallTree];
+    int32_t child[kSmallTree][8];
+    uint32_t idx[kSmallTree], head_id[kSmallTree];
+    int32_t left[kSmallTree], right[kSmallTree], parent[kSmallTree], delta[kSmallTree];
+    int32_t meta[kSmallTree], opar[kSmallTree], pending[kSmallTree];
+    double red[7][32], root[4];
+    uint32_t scan[33], most_bits, depth;
+    int32_t root_done;
+};
+
+// Sorts (a, b, id) over the block, one triple per thread, ascending (b only with kTwo):
+// a bitonic network, through shared memory where partners are in other warps.
+template <bool kTwo>
+__device__ inline void small_sort(uint64_t &a, uint64_t &b, uint32_t &id, SmallTree &s) {
+    const unsigned FULL = 0xffffffffu;
+    const uint32_t t = threadIdx.x;
+    for (uint32_t size = 2; size <= blockDim.x; size <<= 1) {
+        for (uint32_t stride = size >> 1; stride > 0; stride >>= 1) {
+            uint64_t pa, pb = 0;
+            uint32_t pid;
+            if (stride < 32) {
+                pa = __shfl_xor_sync(FULL, a, stride);
+                if constexpr (kTwo) pb = __shfl_xor_sync(FULL, b, stride);
+                pid = __shfl_xor_sync(FULL, id, stride);
+            } else {
+                s.k1[t] = a;
+                if constexpr (kTwo) s.k2[t] = b;
+                s.idx[t] = id;
+                __syncthreads();
+                pa = s.k1[t ^ stride];
+                if constexpr (kTwo) pb = s.k2[t ^ stride];
+                pid = s.idx[t ^ stride];
+                __syncthreads();
+            }
+            const bool low = ((t & stride) == 0) == ((t & size) == 0);  // keeps the smaller
+            bool less = pa < a;
+            if (pa == a) less = kTwo ? pb < b || (pb == b && pid < id) : pid < id;
+            if (less == low) {
+                a = pa;
+                b = pb;
+                id = pid;
+            }
+        }
+    }
+    s.k1[t] = a;
+    if constexpr (kTwo) s.k2[t] = b;
+    s.idx[t] = id;
+    __syncthreads();
+}
+
+template <typename T>
+__global__ void __launch_bounds__(kSmallTree)
+    k_small_tree(const double *__restrict__ pos, const double *__restrict__ vel, const double *__restrict__ mass, uint32_t n,
+                 int keep_root, int reset, uint32_t *__restrict__ sidx, double4 *__restrict__ body,
+                 double4 *__restrict__ onode, int32_t *__restrict__ ochild, int32_t *__restrict__ ometa,
+                 int32_t *__restrict__ oparent, int32_t *__restrict__ leaf_oparent, DevScalars *sc) {
+    extern __shared__ __align__(16) unsigned char small_raw[];
+    SmallTree &s = *reinterpret_cast<SmallTree *>(small_raw);
+    griddep();
+    constexpr bool single = sizeof(T) == 4;
+    const uint32_t t = threadIdx.x;
+    const int lane = t & 31, wid = t >> 5, nw = blockDim.x >> 5;
+    const bool mine = t < n;
+    // ---- root cube, as k_bbox
+    double v[7] = {INFINITY, INFINITY, INFINITY, INFINITY, INFINITY, INFINITY, -0.0};
+    double p[3] = {0.0, 0.0, 0.0};
+    uint32_t bad = 0;
+    if (mine) {
+        double4 b = make_double4(pos[3 * t], pos[3 * t + 1], pos[3 * t + 2], mass[t]);
+        bad = !(isfinite(b.x) && isfinite(b.y) && isfinite(b.z) && isfinite(b.w));
+        p[0] = b.x; p[1] = b.y; p[2] = b.z;
+        v[0] = b.x; v[1] = b.y; v[2] = b.z; v[3] = -b.x; v[4] = -b.y; v[5] = -b.z;
+        if (vel) {
+            const double vx = vel[3 * t], vy = vel[3 * t + 1], vz = vel[3 * t + 2];
+            v[6] = -(vx * vx + vy * vy + vz * vz);
+        }
+        if (single) {
+            b.x = (double)__double2float_rn(b.x); b.y = (double)__double2float_rn(b.y);
+            b.z = (double)__double2float_rn(b.z); b.w = (double)__double2float_rn(b.w);
+        }
+        s.node[t] = b;  // in user order, until the nodes need the room
+        leaf_oparent[t] = -1;
+    }
+    for (int k = 0; k < 7; k++) {
+        const double r = warp_min(v[k]);
+        if (lane == 0) s.red[k][wid] = r;
+    }
+    if (t == 0) {
+        s.most_bits = 0u;
+        s.depth = 0u;
+        s.root_done = 0;
+        if (reset) reset_pass(sc);
+    }
+    bad = __syncthreads_or(bad);
+    if (wid == 0) {
+        double r[7];
+        for (int k = 0; k < 7; k++) r[k] = warp_min(lane < nw ? s.red[k][lane] : INFINITY);
+        if (lane == 0) {
+            if (bad) atomicOr(&sc->status, kStatusNonFinite);
+            if (!keep_root) {
+                const double lo[3] = {r[0], r[1], r[2]}, hi[3] = {-r[3], -r[4], -r[5]};
+                for (int k = 0; k < 3; k++) {
+                    sc->bbox_min[k] = lo[k];
+                    sc->bbox_max[k] = hi[k];
+                }
+                double center[3], side;
+                root_from_extrema(lo, hi, single, center, &side);
+                for (int k = 0; k < 3; k++) sc->root_center[k] = center[k];
+                sc->root_side = side;
+            }
+            sc->max_vel_bits = (unsigned long long)__double_as_longlong(sqrt(-r[6]));
+            for (int k = 0; k < 3; k++) s.root[k] = sc->root_center[k];
+            s.root[3] = sc->root_side;
+        }
+    }
+    __syncthreads();
+    // ---- keys and order: by the first word, then, where two agree, by both
+    uint64_t w[2] = {~0ull, ~0ull};
+    uint32_t id = t;
+    if (mine) descend_words<T>(p, s.root, 1, w);
+    small_sort<false>(w[0], w[1], id, s);
+    bool tie = t + 1 < n && s.k1[t] == s.k1[t + 1];
+    if (__syncthreads_or(tie)) {
+        w[1] = ~0ull;
+        if (mine) {  // (the first n places hold the particles)
+            const double4 b = s.node[id];
+            const double q[3] = {b.x, b.y, b.z};
+            descend_words<T>(q, s.root, 2, w);
+        }
+        small_sort<true>(w[0], w[1], id, s);
+        tie = t + 1 < n && s.k1[t] == s.k1[t + 1] && s.k2[t] == s.k2[t + 1];
+    } else {
+        tie = false;
+    }
+    if (mine) s.body[t] = s.node[id];
+    if (__syncthreads_or(tie)) {
+        deep_group_at(t, s.k1, s.k2, s.k3, s.idx, s.body, n, nullptr, nullptr, s.root, sc, single);
+        __syncthreads();
+    }
+    if (mine) {
+        sidx[t] = s.idx[t];
+        body[t] = s.body[t];
+    }
+    if (n < 2) return;
+    // ---- binary radix tree
+    const int m = (int)n - 1, i = (int)t;
+    const KeyView kv{s.k1, s.k2, s.k3, (int)n, nullptr};
+    const bool node = i < m;
+    if (node) {
+        const int dn = kv.delta(i, i + 1);
+        atomicMax(&s.most_bits, (uint32_t)dn + 1u);
+        int left, right;
+        s.delta[i] = radix_node(kv, i, dn, left, right);
+        s.left[i] = left;
+        s.right[i] = right;
+        if (left >= 0) s.parent[left] = i;
+        if (right >= 0) s.parent[right] = i;
+        if (i == 0) s.parent[0] = -1;
+        s.opar[i] = -1;
+    }
+    __syncthreads();
+    // ---- octree heads, numbered, and their children
+    bool head = false;
+    if (node) {
+        const int q = s.parent[i];
+        head = q < 0 || level_of(s.delta[q]) < level_of(s.delta[i]);
+    }
+    uint32_t nodes;
+    const uint32_t number = block_exclusive_scan(head ? 1u : 0u, s.scan, &nodes);
+    if (node) s.head_id[i] = number;
+    __syncthreads();
+    if (head) {
+        const int L = level_of(s.delta[i]);
+        int nch = 0, nint = 0;
+        collapse_node(i, L, s.left, s.right, s.delta, [&](int ch) {
+            if (nch >= 8) {
+                atomicOr(&sc->status, kStatusCapacity);
+                return;
+            }
+            if (ch < 0) {
+                leaf_oparent[~ch] = (int)number;
+            } else {
+                ch = (int)s.head_id[ch];
+                s.opar[ch] = (int)number;
+                nint++;
+            }
+            s.child[number][nch++] = ch;
+        }, &sc->status);
+        s.meta[number] = L | (nch << 8) | (nint << 12);
+        s.pending[number] = nint;
+        atomicMax(&s.depth, (uint32_t)L);
+    }
+    __syncthreads();
+    // ---- mass and centre of mass: each round, the nodes whose node children are done
+    const bool onod = t < nodes;
+    const int meta = onod ? s.meta[t] : 0, nch = meta_nchild(meta);
+    bool done = !onod;
+    for (int round = 0; round <= kMaxLevels + 1; round++) {
+        const bool now = !done && *(volatile int32_t *)&s.pending[t] == 0;
+        if (now) {
+            s.node[t] = node_com<T>(
+                meta_level(meta), nch, [&](int k) { return s.child[t][k]; }, [&](int j) { return s.body[j]; },
+                [&](int c, double &cm, int &level) {
+                    const double4 q = s.node[c];
+                    cm = q.w;
+                    level = meta_level(s.meta[c]);
+                    return make_double3(q.x, q.y, q.z);
+                });
+            done = true;
+        }
+        __syncthreads();
+        if (now) {
+            const int up = s.opar[t];
+            if (up >= 0) atomicSub(&s.pending[up], 1);
+            else s.root_done = 1;
+        }
+        __syncthreads();
+        if (s.root_done) break;
+    }
+    if (onod) {
+        if (!done) atomicOr(&sc->status, kStatusCapacity);  // (never in a well-formed tree)
+        onode[t] = s.node[t];
+        ometa[t] = meta;
+        oparent[t] = s.opar[t];
+        for (int k = 0; k < nch; k++) ochild[8 * (size_t)t + k] = s.child[t][k];
+    }
+    if (t == 0) {
+        sc->n_onodes = nodes;
+        sc->depth = s.depth;
+        sc->max_prefix_bits = s.most_bits;
+    }
+}
+
+cudaError_t small_tree(const TreeBuild &tb, cudaStream_t st) {
+    unsigned threads = 64;
+    while (threads < tb.n) threads <<= 1;
+    auto *k = tb.single ? k_small_tree<float> : k_small_tree<double>;
+    const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SmallTree));
+    if (e != cudaSuccess) return e;
+    return launch_pdl(k, dim3(1), dim3(threads), sizeof(SmallTree), st, tb.pos, tb.vel_for_max, tb.mass, tb.n, tb.keep_root,
+                      tb.reset, tb.idx_a, tb.body, tb.onode, tb.ochild, tb.ometa, tb.oparent, tb.leaf_oparent, tb.sc);
+}
+
+// ---------------------------------------------------------------------------
 static inline unsigned blocks_for(uint64_t n, unsigned t) { return (unsigned)((n + t - 1) / t); }
 
 cudaError_t build_octree(const TreeBuild &tb, cudaStream_t st, unsigned *launches) {
@@ -958,6 +1240,11 @@ cudaError_t build_octree(const TreeBuild &tb, cudaStream_t st, unsigned *launche
     unsigned L = 0;
     if (n == 0) return tb.reset ? launch_reset_pass(tb.sc, st) : cudaSuccess;
     const bool multi = tb.nsys > 1;
+    if (is_small_tree(tb)) {
+        if (tb.mass_ready) cudaStreamWaitEvent(st, tb.mass_ready, 0);
+        *launches += 1;
+        return small_tree(tb, st);
+    }
     // The plan's passes: on the second word, on the first, or (several systems) on the
     // system's number and the first word together.
     const int p2 = multi ? 0 : tb.sort_p2, p1 = multi ? 0 : tb.sort_p1, pm = multi ? tb.sort_pm : 0;
@@ -1072,7 +1359,7 @@ cudaError_t build_octree(const TreeBuild &tb, cudaStream_t st, unsigned *launche
 
 cudaError_t compute_com(const TreeBuild &tb, cudaStream_t st, unsigned *launches) {
     const uint32_t n = tb.n;
-    if (n < 2) return cudaSuccess;
+    if (n < 2 || is_small_tree(tb)) return cudaSuccess;  // (a small system's build has done it)
     // (the arrival counts were zeroed by the build's k_head_flags)
     const bool groups = n <= kComGroupsMax;
     const dim3 grid(blocks_for((uint64_t)(n - 1) * (groups ? kComLanes : 1), 256));

@@ -55,6 +55,11 @@ struct TreeBuild {
     int32_t *sys_root_node;      // octree root of each system (-1: fewer than 2 particles)
 };
 
+// Systems up to this size (a single one) are built by one block, masses and centres of
+// mass included, without a sort plan.
+constexpr uint32_t kSmallTree = 1024;
+inline bool is_small_tree(const TreeBuild &tb) { return tb.nsys <= 1 && tb.n <= kSmallTree; }
+
 // Enqueues root cube -> keys -> sort -> bodies -> radix tree -> octree.
 cudaError_t build_octree(const TreeBuild &tb, cudaStream_t st, unsigned *launches);
 // Enqueues the bottom-up mass / centre-of-mass pass.

@@ -484,8 +484,8 @@ int force_pass(nbody_ctx *c, int damping, double theta, bool fp64, bool want_vma
 // Clears the per-call status bits and the per-call interaction total.
 int begin_call(nbody_ctx *c) {
     c->call++;
-    NB_CUDA(cudaMemsetAsync(&c->sc->status, 0, sizeof(uint32_t), c->stream));
-    NB_CUDA(cudaMemsetAsync(&c->sc->interactions_total, 0, sizeof(unsigned long long), c->stream));
+    constexpr size_t at = offsetof(DevScalars, interactions_total), end = offsetof(DevScalars, status) + sizeof(uint32_t);
+    NB_CUDA(cudaMemsetAsync((char *)c->sc + at, 0, end - at, c->stream));
     return NBODY_OK;
 }
 

@@ -80,12 +80,13 @@ struct DevScalars {
     double bbox_min[3];
     double bbox_max[3];
     unsigned long long interactions;
-    unsigned long long interactions_total;  // summed over the steps of one API call
     unsigned long long walk_entries;        // node entries the walk warps tested (union lists)
     unsigned long long walk_tiles;          // stack tiles the walk warps staged
     unsigned long long walk_decisions;      // internal nodes decided by a warp
     unsigned long long walk_list;           // bodies entered in the warps' interaction lists
     unsigned long long walk_near;           // bodies taken with FP64 offsets (near the group box)
+    // zeroed together when an API call begins
+    unsigned long long interactions_total;  // summed over the steps of one API call
     uint32_t status;
     uint32_t n_onodes;
     uint32_t depth;

@@ -65,17 +65,21 @@ struct GroupConsts {
     uint32_t st[6];     // per-group statistics: entries, tiles, decisions, list, near, longest queue
 };
 
+// Floats from one pair of mixed nodes to the next: 20 and not 16, so that the stores of
+// a tile's pairs spread over 16 banks instead of 4 (1M bodies: -0.8% walk time).
+constexpr int kPair = 20;
+
 // Shared memory of one warp: the tile's nodes that are decided lane by lane.
 template <bool kFp64>
 struct TileSmem;
 template <>
 struct TileSmem<false> {
     // The tile's mixed nodes, compacted and stored in pairs: pair j holds
-    // x0 x1 y0 y1 z0 z1 -q0 -q1 band0 band1 reach0 reach1 ref0 ref1 - - at 16 j
+    // x0 x1 y0 y1 z0 z1 -q0 -q1 band0 band1 reach0 reach1 ref0 ref1 - - at kPair j
     // ((com - ref).xyz, q = (side/theta)^2, the half-width of its error band, the
     // mask of lanes that reached the node, the node). Once a pair is decided,
     // its first two words hold the two open masks.
-    alignas(16) float mx[16 * 16];
+    alignas(16) float mx[16 * kPair];
 };
 template <>
 struct TileSmem<true> {
@@ -536,6 +540,15 @@ __device__ inline void sum_batch(G &s, int start, int count, int lane, const Wal
 // waiting entries the newest go first, one tile at a time, which bounds the queue;
 // a team takes no more tiles at once than keep the order of one warp's walk.)
 //
+// Nodes, bodies and children are gathered, one 32-byte load each. Many groups keep the
+// load pipe of the L1 and shared memory at 76% beside 69% of the issue slots (1M bodies,
+// with two 16-byte loads each), so there a node's children are loaded once it is known
+// that it is opened, as about one in three is: 981 to 946 us, and 931 with 32-byte loads;
+// a collapsed system 3585 to 3470 and 3415. The other forms wait for their loads instead
+// (teams) or have too few warps an SM to cover a second one (FP64, adjoint) and take the
+// children along with the node (20,011 bodies: 53 us, 56 with the later load; FP64 of
+// 200,000: 1117, 1150; adjoint of 100,000: 629, 693).
+//
 // Bound of few groups: the serial chain of one group's tiles (~3 us each at one warp
 // per scheduler; 11% of issue slots used on a shell of 20,011), which a team of four
 // cuts to a third; of many: instruction issue (67% of slots), where one warp each
@@ -553,6 +566,7 @@ __global__ void __launch_bounds__((kTeam ? kTeamMaxWarps : kWalkMaxWarps) * 32) 
     constexpr int kLists = kFp64 ? 1 : kAdj ? 2 : 3;
     constexpr int NC = kPot ? 4 : 3;
     constexpr uint32_t kCap = kTeam ? kTeamList : kSoloList;
+    constexpr bool kLate = !kTeam && !kFp64 && !kAdj;  // children loaded for opened nodes only
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     Team &tm = *reinterpret_cast<Team *>(smem_raw);
     Solo &solo = reinterpret_cast<Solo *>(smem_raw)[kTeam ? 0 : wid];
@@ -717,17 +731,15 @@ __global__ void __launch_bounds__((kTeam ? kTeamMaxWarps : kWalkMaxWarps) * 32) 
                 ref = e.x;
                 reach = (uint32_t)e.y;
                 if (ref >= 0) {
-                    const double4 nd = t.onode[ref];
+                    const double4 nd = load32(t.onode + ref);
                     const int meta = t.ometa[ref];
                     cx = nd.x; cy = nd.y; cz = nd.z; m = nd.w;
                     nch = meta_nchild(meta);
                     so = exp2_neg(meta_level(meta));  // 2^-level
-                    const int4 *cp = reinterpret_cast<const int4 *>(t.ochild + 8 * (size_t)ref);
-                    ch0 = cp[0];
-                    ch1 = cp[1];
+                    if constexpr (!kLate) load32(t.ochild + 8 * (size_t)ref, ch0, ch1);
                     is_int = true;
                 } else {
-                    const double4 bd = t.body[~ref];
+                    const double4 bd = load32(t.body + ~ref);
                     cx = bd.x; cy = bd.y; cz = bd.z; m = bd.w;
                     const uint32_t own = (uint32_t)(~ref) - g0;  // a leaf of this group: not its own lane
                     if (own < 32u) reach &= ~(1u << own);
@@ -824,13 +836,13 @@ __global__ void __launch_bounds__((kTeam ? kTeamMaxWarps : kWalkMaxWarps) * 32) 
                     const int nmix = __popc(intm);
                     const int mpos = __popc(intm & lt);
                     if (mixed) {
-                        float *e = tile.mx + 16 * (mpos >> 1) + (mpos & 1);
+                        float *e = tile.mx + kPair * (mpos >> 1) + (mpos & 1);
                         e[0] = fcx; e[2] = fcy; e[4] = fcz; e[6] = -qf;
                         e[8] = band; e[10] = __uint_as_float(reach); e[12] = __int_as_float(ref);
                     }
                     if (lane == 0 && (nmix & 1)) {
                         // pad an odd count with an entry no lane reached
-                        float *e = tile.mx + 16 * (nmix >> 1) + 1;
+                        float *e = tile.mx + kPair * (nmix >> 1) + 1;
                         e[0] = 0.f; e[2] = 0.f; e[4] = 0.f; e[6] = 0.f;
                         e[8] = 0.f; e[10] = 0.f; e[12] = 0.f;
                     }
@@ -839,7 +851,7 @@ __global__ void __launch_bounds__((kTeam ? kTeamMaxWarps : kWalkMaxWarps) * 32) 
                     const uint64_t npx = f2pack(-px, -px), npy = f2pack(-py, -py), npz = f2pack(-pz, -pz);
                     const uint32_t bit = 1u << lane;
                     for (int k = 0; k < nmix; k += 2) {
-                        float *pr = tile.mx + 8 * k;
+                        float *pr = tile.mx + (kPair / 2) * k;
                         const float4 A = *reinterpret_cast<const float4 *>(pr);      // x0 x1 y0 y1
                         const float4 B = *reinterpret_cast<const float4 *>(pr + 4);  // z0 z1 -q0 -q1
                         const float4 C = *reinterpret_cast<const float4 *>(pr + 8);  // band0 band1 reach0 reach1
@@ -878,7 +890,7 @@ __global__ void __launch_bounds__((kTeam ? kTeamMaxWarps : kWalkMaxWarps) * 32) 
                         if (lane == 0) *reinterpret_cast<uint2 *>(pr) = make_uint2(om1, om2);
                     }
                     __syncwarp();
-                    if (mixed) my_open = __float_as_uint(tile.mx[16 * (mpos >> 1) + (mpos & 1)]);
+                    if (mixed) my_open = __float_as_uint(tile.mx[kPair * (mpos >> 1) + (mpos & 1)]);
                 }
                 __syncwarp();
             }
@@ -910,6 +922,7 @@ __global__ void __launch_bounds__((kTeam ? kTeamMaxWarps : kWalkMaxWarps) * 32) 
             const uint32_t nmk = !kFp64 ? __ballot_sync(FULL, near) : 0u;
             // exclusive prefix of the child counts (0..8) from four independent ballots of their bits
             const int myn = my_open ? nch : 0;
+            if (kLate && myn > 0) load32(t.ochild + 8 * (size_t)ref, ch0, ch1);
             const uint32_t q0 = __ballot_sync(FULL, myn & 1), q1 = __ballot_sync(FULL, myn & 2),
                            q2 = __ballot_sync(FULL, myn & 4), q3 = __ballot_sync(FULL, myn & 8);
             const uint32_t pre = __popc(q0 & lt) + 2 * __popc(q1 & lt) + 4 * __popc(q2 & lt) + 8 * __popc(q3 & lt);

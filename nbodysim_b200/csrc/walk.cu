@@ -93,10 +93,10 @@ struct TileSmem<true> {
 //   MIXED forward: entries every lane takes, entries some lanes take (a lane mask
 //   each), and bodies near the group's box; MIXED adjoint: the last two; FP64: one,
 //   with masks.
-// MIXED forward lists are stored in pairs of entries, so that the packed FP32
+// MIXED lists are stored in pairs of entries, so that the packed FP32
 // instructions (two lanes of arithmetic each) read their operands straight from
 // two 16-byte loads: entries 2j and 2j+1 occupy 8 floats
-// (x0, x1, y0, y1, z0, z1, Gm0, Gm1) at 8j. The adjoint keeps one float4 per entry.
+// (x0, x1, y0, y1, z0, z1, Gm0, Gm1) at 8j. The adjoint's near list is FP64.
 template <bool kFp64, bool kAdj, int kCap>
 struct GroupSmem;
 
@@ -114,9 +114,10 @@ struct GroupSmem<false, false, kCap> {
 template <int kCap>
 struct GroupSmem<false, true, kCap> {
     GroupConsts gc;
-    alignas(16) float4 lc[kCap];      // (com - ref).xyz, G m
+    alignas(16) float lp[4 * kCap];
     alignas(16) double4 nc[kCap];     // near: com.xyz (absolute), G m
-    uint32_t lm[kCap], nm[kCap];
+    alignas(8) uint32_t lm[kCap];
+    uint32_t nm[kCap];
     int lr[kCap], nr[kCap];           // node refs
     float acc[2][3][32];
 };
@@ -380,31 +381,78 @@ __device__ inline void scatter_adj8(double *adj_node, double *adj_leaf, const in
 }
 
 // The list in chunks of eight entries: every lane's pair terms for the chunk,
-// one transposed warp reduction, one atomic per lane.
+// one transposed warp reduction, one atomic per lane. The terms are those of
+// pair_adjoint, without damping two entries per packed instruction, where an entry not
+// taken enters with inverse distance 0, which makes every one of its terms 0. What is
+// missing of the last chunk is padded with far, massless entries that no lane takes.
+//
+// Bound: instruction issue, most of it these terms and the reduction (125 a chunk).
+// Packed terms: adjoint walk of 65,536 bodies 470 to 435 us, 100,000 633 to 582,
+// 500,000 2600 to 2300 (5000, where a team waits for one group's chain: 90 to 92;
+// damped 65,536, whose terms are the scalar ones as before: 880 and 894).
 template <bool kDamp>
-__device__ inline void adj_list_f32(const float4 *lc, const uint32_t *lm, const int *lr, int count, int lane,
-                                    float px, float py, float pz, float lax, float lay, float laz, float &gx,
-                                    float &gy, float &gz, double *adj_node, double *adj_leaf) {
+__device__ inline void adj_list_f32(float *l, uint32_t *lm, const int *lr, int count, int lane, float px, float py,
+                                    float pz, float lax, float lay, float laz, float &gx, float &gy, float &gz,
+                                    double *adj_node, double *adj_leaf) {
+    if (count & 7) {
+        const int k = count + lane;
+        __syncwarp();
+        if (k < ((count + 7) & ~7)) {
+            put_pair_entry(l, k, 1e18f, 1e18f, 1e18f, 0.f);
+            lm[k] = 0u;
+        }
+        __syncwarp();
+    }
+    const uint32_t bit = 1u << lane;
+    const uint64_t npx = f2pack(-px, -px), npy = f2pack(-py, -py), npz = f2pack(-pz, -pz);
+    const uint64_t lx = f2pack(lax, lax), ly = f2pack(lay, lay), lz = f2pack(laz, laz);
+    const uint64_t g2 = f2pack((float)kG, (float)kG);
+    uint64_t sx = f2pack(0.f, 0.f), sy = sx, sz = sx;
     for (int k0 = 0; k0 < count; k0 += 8) {
         float v[32];
 #pragma unroll
-        for (int j = 0; j < 8; j++) {
-            const int k = k0 + j;
-            float vx = 0.f, vy = 0.f, vz = 0.f, mt = 0.f;
-            if (k < count) {
-                const float4 c = lc[k];
-                const bool take = (lm[k] >> lane) & 1u;
-                const float dx = c.x - px, dy = c.y - py, dz = c.z - pz;
-                const float r2 = fmaf(dz, dz, fmaf(dy, dy, dx * dx));
-                pair_adjoint<kDamp, float>(dx, dy, dz, r2, c.w, lax, lay, laz, vx, vy, vz, mt);
-                if (!take) vx = vy = vz = mt = 0.f;
+        for (int j = 0; j < 8; j += 2) {
+            const float4 A = *reinterpret_cast<const float4 *>(l + 4 * (k0 + j));      // x0 x1 y0 y1
+            const float4 B = *reinterpret_cast<const float4 *>(l + 4 * (k0 + j) + 4);  // z0 z1 g0 g1
+            const uint2 m = *reinterpret_cast<const uint2 *>(lm + k0 + j);
+            if constexpr (kDamp) {  // an exponential and three divides an entry: nothing to gain by packing
+#pragma unroll
+                for (int h = 0; h < 2; h++) {
+                    float *w = v + 4 * (j + h);
+                    const float dx = (h ? A.y : A.x) - px, dy = (h ? A.w : A.z) - py, dz = (h ? B.y : B.x) - pz;
+                    const float r2 = fmaf(dz, dz, fmaf(dy, dy, dx * dx));
+                    pair_adjoint<true, float>(dx, dy, dz, r2, h ? B.w : B.z, lax, lay, laz, w[0], w[1], w[2], w[3]);
+                    if (!((h ? m.y : m.x) & bit)) w[0] = w[1] = w[2] = w[3] = 0.f;
+                    gx -= w[0]; gy -= w[1]; gz -= w[2];
+                }
+            } else {
+                const uint64_t dx = f2add(f2pack(A.x, A.y), npx), dy = f2add(f2pack(A.z, A.w), npy),
+                               dz = f2add(f2pack(B.x, B.y), npz);
+                const uint64_t r2 = f2fma(dz, dz, f2fma(dy, dy, f2mul(dx, dx)));
+                float r0, r1;
+                f2unpack(r2, r0, r1);
+                const uint64_t inv = f2pack((m.x & bit) ? rsqrt_ftz(r0) : 0.f, (m.y & bit) ? rsqrt_ftz(r1) : 0.f);
+                const uint64_t ux = f2mul(dx, inv), uy = f2mul(dy, inv), uz = f2mul(dz, inv);
+                const uint64_t sh = f2fma(uz, lz, f2fma(uy, ly, f2mul(ux, lx)));
+                const uint64_t gr = f2mul(inv, inv), g = f2mul(gr, inv);
+                const uint64_t gm = f2pack(B.z, B.w), c = f2mul(f2mul(g, f2pack(-3.f, -3.f)), sh);
+                const uint64_t vx = f2mul(gm, f2fma(c, ux, f2mul(g, lx))), vy = f2mul(gm, f2fma(c, uy, f2mul(g, ly))),
+                               vz = f2mul(gm, f2fma(c, uz, f2mul(g, lz)));
+                const uint64_t mt = f2mul(f2mul(g2, gr), sh);
+                sx = f2add(sx, vx); sy = f2add(sy, vy); sz = f2add(sz, vz);
+                f2unpack(vx, v[4 * j], v[4 * j + 4]);
+                f2unpack(vy, v[4 * j + 1], v[4 * j + 5]);
+                f2unpack(vz, v[4 * j + 2], v[4 * j + 6]);
+                f2unpack(mt, v[4 * j + 3], v[4 * j + 7]);
             }
-            gx -= vx; gy -= vy; gz -= vz;
-            v[4 * j] = vx; v[4 * j + 1] = vy; v[4 * j + 2] = vz; v[4 * j + 3] = mt;
         }
         const float z = warp_transpose_sum32(v, lane);
         scatter_adj8(adj_node, adj_leaf, lr, k0, count, (double)z, lane);
     }
+    float a0, a1;
+    f2unpack(sx, a0, a1); gx -= a0 + a1;
+    f2unpack(sy, a0, a1); gy -= a0 + a1;
+    f2unpack(sz, a0, a1); gz -= a0 + a1;
 }
 
 template <bool kDamp>
@@ -506,7 +554,7 @@ __device__ inline void sum_batch(G &s, int start, int count, int lane, const Wal
         if (a.counts) cnt += count_list(s.lm + start, count, bit);
     } else if constexpr (kAdj) {
         if constexpr (kList == 0) {
-            adj_list_f32<kDamp>(s.lc + start, s.lm + start, s.lr + start, count, lane, px, py, pz, (float)lax,
+            adj_list_f32<kDamp>(s.lp + 4 * start, s.lm + start, s.lr + start, count, lane, px, py, pz, (float)lax,
                                 (float)lay, (float)laz, v[0], v[1], v[2], a.adj_node, a.adj_leaf);
             if (a.counts) cnt += count_list(s.lm + start, count, bit);
         } else {
@@ -959,7 +1007,7 @@ __global__ void __launch_bounds__((kTeam ? kTeamMaxWarps : kWalkMaxWarps) * 32) 
             } else if constexpr (kAdj) {
                 if (take_it) {
                     const int pos = slot_of(0, off_p, pmk);
-                    s.lc[pos] = make_float4(fcx, fcy, fcz, (float)(kG * m));
+                    put_pair_entry(s.lp, pos, fcx, fcy, fcz, (float)(kG * m));
                     s.lm[pos] = accm;
                     s.lr[pos] = ref;
                 } else if (near) {

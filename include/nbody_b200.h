@@ -51,7 +51,7 @@ extern "C" {
 #define NBODY_ERR_COINCIDENT 4   /* two particles agree on all 63 octree levels; the reference
                                     recurses without bound on such input (src/octree.cpp:173-195) */
 #define NBODY_ERR_NONFINITE 5    /* a position or mass is NaN or infinite */
-#define NBODY_ERR_CAPACITY 6     /* a walk's node stack exceeded its spill capacity */
+#define NBODY_ERR_CAPACITY 6     /* the octree or a walk's queue of nodes exceeded its capacity */
 #define NBODY_ERR_NO_DEVICE 7    /* no CUDA device, or the device is not sm_100 */
 #define NBODY_ERR_STATE 8        /* call out of order (e.g. step before particles are set) */
 
@@ -158,7 +158,7 @@ typedef struct nbody_stats {
     /* walk_entries .. walk_near and max_stack: collected only while
      * nbody_set_walk_stats(ctx, 1) is on (0 otherwise) */
     uint64_t walk_entries;       /* node entries tested by the walk's warps in the last pass */
-    uint64_t walk_tiles;         /* stack tiles (<= 32 entries) the walk's warps staged */
+    uint64_t walk_tiles;         /* tiles (<= 32 queued nodes) the walk's warps staged */
     uint64_t walk_decisions;     /* internal nodes the warps decided (open / accept) */
     uint64_t walk_list;          /* bodies the warps put in their interaction lists */
     uint64_t walk_near;          /* bodies taken with FP64 offsets (too close for FP32 offsets) */
@@ -166,7 +166,7 @@ typedef struct nbody_stats {
     uint32_t walk_blocks;          /* walk grid size in use (persistent blocks) */
     uint32_t tree_nodes;     /* internal nodes of the (chain-free) octree */
     uint32_t tree_depth;     /* deepest internal-node level */
-    uint32_t max_stack;      /* deepest walk stack seen (entries) */
+    uint32_t max_stack;      /* longest queue of nodes a walk held (entries) */
     uint32_t fallback_tests; /* opening tests settled by the exact FP64 path */
     double last_dt;          /* dt used by the last step */
     double root_center[3];

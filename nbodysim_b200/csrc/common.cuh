@@ -94,7 +94,7 @@ struct DevScalars {
     double bbox_max[3];
     unsigned long long interactions;
     unsigned long long walk_entries;        // node entries the walk warps tested (union lists)
-    unsigned long long walk_tiles;          // stack tiles the walk warps staged
+    unsigned long long walk_tiles;          // tiles of queued nodes the walk warps staged
     unsigned long long walk_decisions;      // internal nodes decided by a warp
     unsigned long long walk_list;           // bodies entered in the warps' interaction lists
     unsigned long long walk_near;           // bodies taken with FP64 offsets (near the group box)

@@ -5,7 +5,7 @@
 // leaf, otherwise it accepts the node unless the node is its own leaf; an
 // accepted node adds G M (com - x) / r^3 (src/main.cpp:306-333). Every lane
 // keeps exactly its own decisions: the warp walks the union of the 32 walks,
-// carrying with every stacked node the mask of lanes that reached it (opened
+// carrying with every queued node the mask of lanes that reached it (opened
 // all its ancestors). Lanes outside the mask ignore the node, so each lane's
 // accepted set is the reference's set for that particle.
 //
@@ -130,7 +130,7 @@ struct GroupSmem<true, kAdj, kCap> {
     double acc[1][4][32];             // x, y, z, potential
 };
 
-// A team's block: its group, the queue, the batches summed in this round, and what
+// A team's block: its group, the queue, the batches summed in one turn, and what
 // each warp's tile adds.
 constexpr int kTeamSlots = kTeamMaxWarps + 3;
 template <bool kFp64, bool kAdj>
@@ -599,7 +599,7 @@ __device__ inline void sum_batch(G &s, int start, int count, int lane, const Wal
 //
 // Bound of few groups: the serial chain of one group's tiles (~3 us each at one warp
 // per scheduler; 11% of issue slots used on a shell of 20,011), which a team of four
-// cuts to a third; of many: instruction issue (67% of slots), where one warp each
+// cuts to a third; of many: instruction issue (73% of slots), where one warp each
 // needs no barriers. Teams of 2, 6 and 8 warps were slower (5000 particles: 79, 51,
 // 55 us against 51 with four; 65,536: 291, 330, 446 against 258). A stack cut into
 // parts for several warps, last in first out, was as fast for few groups, but one

@@ -51,7 +51,7 @@ extern "C" {
 #define NBODY_ERR_COINCIDENT 4   /* two particles agree on all 63 octree levels; the reference
                                     recurses without bound on such input (src/octree.cpp:173-195) */
 #define NBODY_ERR_NONFINITE 5    /* a position or mass is NaN or infinite */
-#define NBODY_ERR_CAPACITY 6     /* the octree or a walk's queue of nodes exceeded its capacity */
+#define NBODY_ERR_CAPACITY 6     /* the octree exceeded its capacity (it is then not walked) */
 #define NBODY_ERR_NO_DEVICE 7    /* no CUDA device, or the device is not sm_100 */
 #define NBODY_ERR_STATE 8        /* call out of order (e.g. step before particles are set) */
 

@@ -608,6 +608,10 @@ template <bool kFp64, bool kDamp, bool kPot, bool kAdj, bool kStats, bool kTeam>
 __global__ void __launch_bounds__((kTeam ? kTeamMaxWarps : kWalkMaxWarps) * 32) k_walk(WalkArgs a) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     griddep();
+    // A walk ends, within its queue, on a well-formed octree only. Where the build has
+    // reported that it is not (a sort that gave up, a node with too many children), the
+    // pass stops here and the host reports the error.
+    if (a.t.sc->status & (kStatusSortStall | kStatusCapacity)) return;
     using Acc = std::conditional_t<kFp64, double, float>;
     using Team = TeamSmem<kFp64, kAdj>;
     using Solo = SoloSmem<kFp64, kAdj>;

@@ -20,9 +20,7 @@ __device__ inline double approx_inverse(double r2, double &e) {
 
 // Within plain_range: the approximation corrected by the binomial series of
 // (1 - e)^(-1/2) = 1 + 1/2 e + 3/8 e^2 + ..., or, in the cube, of (1 - e)^(-3/2) =
-// 1 + 3/2 e + 15/8 e^2 + ...; the next terms are below 2^-58. A direct sum's pair force
-// with inverse_cube has a root mean square error of 1.52e-16 against an 80-bit one
-// (with a square root and divides: 1.57e-16).
+// 1 + 3/2 e + 15/8 e^2 + ...; the next terms are below 2^-58.
 __device__ inline double inverse_root(double r2) {
     double e;
     const double y = approx_inverse(r2, e);

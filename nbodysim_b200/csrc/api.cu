@@ -285,7 +285,8 @@ void next_sort_plan(nbody_ctx *c, const DevScalars &h) {
 
 // The next build's plan for several systems: passes over the top bits of the
 // system's number and the first word together (at most 8; what these leave tied is
-// sorted in place), by the rules above, or the full sort.
+// sorted in place), by the rules above, or the full sort. A plan covers the whole
+// number: pairs across systems are not binned, so the bins cannot ask for it.
 void next_systems_plan(nbody_ctx *c, const DevScalars &h) {
     if (h.max_prefix_bits == 0) return;
     const uint32_t bits = h.max_prefix_bits + (uint32_t)c->sys_bits;
@@ -294,8 +295,9 @@ void next_systems_plan(nbody_ctx *c, const DevScalars &h) {
     const int covered = bits <= 64 ? (int)(bits + 7) / 8 : 0;
     if (h.word_ties) c->sort_pm_cooldown = kPlanCooldown;
     int want = covered ? covered : c->sort_pm_cooldown == 0 && tied <= tol ? 8 : 0;
+    const int least = (c->sys_bits + 7) / 8;
     if (c->sort_pm_cooldown == 0) {
-        while (want > 1) {
+        while (want > least) {
             tied += h.pair_passes[want];
             if (tied > tol) break;
             want--;

@@ -1300,7 +1300,7 @@ cudaError_t build_octree(const TreeBuild &tb, cudaStream_t st, unsigned *launche
         keys(k0, nullptr, i0, pm, shift);
         passes(k0, k0o, i0, i0o, pm, shift, 0);  // result: idx_a
         gather(tb.key3, tb.key_b, sys_id);
-        s1 = std::max(0, 63 - (8 * pm - tb.sys_bits));
+        s1 = std::min(63, std::max(0, 63 - (8 * pm - tb.sys_bits)));
     } else if (p2 > 0) {
         uint64_t *k0 = (p2 & 1) ? tb.key_b : tb.key_a, *k0o = (p2 & 1) ? tb.key_a : tb.key_b;
         uint32_t *i0 = (p2 & 1) ? tb.idx_b : tb.idx_a, *i0o = (p2 & 1) ? tb.idx_a : tb.idx_b;

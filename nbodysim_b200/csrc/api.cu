@@ -766,7 +766,8 @@ int one_step(nbody_ctx *c) {
 // Steps of one call that pay for capturing the step at once.
 constexpr uint32_t kCaptureSteps = 32;
 
-int run_steps(nbody_ctx *c, uint32_t nsteps) {
+// nsteps of the `in_call` steps that the API call takes.
+int run_steps(nbody_ctx *c, uint32_t nsteps, uint32_t in_call) {
     if (c->use_graphs && !c->timing && !merging(c)) {  // merging changes n: launched step by step
         auto key = graph_key(c, 0);
         const bool seen = key == c->step_seen && c->step_seen_call != c->call;
@@ -774,7 +775,7 @@ int run_steps(nbody_ctx *c, uint32_t nsteps) {
             c->step_seen = key;
             c->step_seen_call = c->call;
         }
-        if ((!c->step_exec || key != c->step_key) && (seen || nsteps >= kCaptureSteps)) {
+        if ((!c->step_exec || key != c->step_key) && (seen || in_call >= kCaptureSteps)) {
             drop_graph(c->step_exec);
             c->step_key.clear();
             if (capture(c, &c->step_exec, &c->step_launches, [&] { return one_step(c); })) c->step_key = key;
@@ -1291,7 +1292,7 @@ int nbody_step(nbody_ctx *c, uint32_t nsteps) {
     int rc = begin_call(c);
     if (rc) return rc;
     if ((rc = maybe_autotune(c))) return rc;
-    rc = run_steps(c, nsteps);
+    rc = run_steps(c, nsteps, nsteps);
     if (rc) return rc;
     if ((rc = copy_scalars_back(c))) return rc;
     return check_status(c);
@@ -1351,12 +1352,12 @@ int nbody_step_host(nbody_ctx *c, uint32_t n, double *pos, double *vel, const do
         }
         NB_CUDA(launch_update(c->pos, c->vel, c->acc, fp64, n, sp, c->sc, c->stream));
         c->launches++;
-        if (nsteps > 1 && (rc = run_steps(c, nsteps - 1))) return rc;
+        if (nsteps > 1 && (rc = run_steps(c, nsteps - 1, nsteps - 1))) return rc;
     } else {
         if ((rc = upload(c, n, pos, vel, mass))) return rc;
         c->have_vel = true;
         if ((rc = begin_call(c))) return rc;
-        if ((rc = run_steps(c, nsteps))) return rc;
+        if ((rc = run_steps(c, nsteps, nsteps))) return rc;
     }
     NB_CUDA(cudaMemcpyAsync(pos, c->pos, 24 * (size_t)n, cudaMemcpyDeviceToHost, c->stream));
     NB_CUDA(cudaMemcpyAsync(vel, c->vel, 24 * (size_t)n, cudaMemcpyDeviceToHost, c->stream));
@@ -1471,7 +1472,7 @@ int nbody_forward_checkpointed(nbody_ctx *c, uint32_t nsteps, uint32_t every) {
         NB_CUDA(cudaMemcpyAsync(ck, c->pos, 8 * N3, cudaMemcpyDeviceToDevice, c->stream));
         NB_CUDA(cudaMemcpyAsync(ck + N3, c->vel, 8 * N3, cudaMemcpyDeviceToDevice, c->stream));
         const uint32_t len = nsteps - k < every ? nsteps - k : every;
-        if ((rc = run_steps(c, len))) return rc;
+        if ((rc = run_steps(c, len, nsteps))) return rc;
     }
     if ((rc = copy_scalars_back(c))) return rc;
     if ((rc = check_status(c))) return rc;

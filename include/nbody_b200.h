@@ -189,7 +189,9 @@ typedef struct nbody_stats {
                                   full sort, the ones that cover sort_split_bits; 16 when a pair
                                   needs a third key word. A call of several steps plans the passes
                                   that cover sort_split_bits. A plan shrinks by two passes or more
-                                  at a time. */
+                                  at a time. 0 for a system of at most 1024 particles. Several
+                                  systems: 18 (the full sort) or at most 8, over the system's number
+                                  and the first key word together. */
 } nbody_stats;
 int nbody_get_stats(nbody_ctx *ctx, nbody_stats *out);
 /* Time phases with CUDA events on the context stream (default off; timed calls

@@ -350,7 +350,7 @@ int check_status(nbody_ctx *c) {
     s.sort_split_bits = h.max_prefix_bits;
     s.sort_tie_runs = h.tie_runs;
     if (is_small_tree(c->tb)) {
-        s.sort_passes = 0;  // sorted within one block; the plans stay
+        s.sort_passes = s.sort_next_passes = 0;  // sorted within one block; the plans stay
     } else if (c->tb.nsys > 1) {
         const int used = c->multi_step_call ? c->sort_deep_pm : c->sort_pm;
         s.sort_passes = used == 0 ? 18u : (uint32_t)used + (h.word_ties ? 18u : 0u);
@@ -392,6 +392,19 @@ void tree_inputs(nbody_ctx *c, uint32_t n, bool want_vmax) {
     tb.reset = 0;
 }
 
+// The systems that a force pass on the state takes it for; true if there are several.
+bool tree_layout(nbody_ctx *c) {
+    const bool multi = c->nsys > 1 && !c->single_pass && c->sys_total == c->n;
+    c->tb.n = c->n;
+    c->tb.nsys = multi ? c->nsys : 1;
+    c->tb.sys_start = c->sys_start;
+    c->tb.sys_id = c->sys_id;
+    c->tb.sys_sorted = c->sys_sorted;
+    c->tb.sys_root = c->sys_root;
+    c->tb.sys_root_node = c->sys_root_node;
+    return multi;
+}
+
 void ev(nbody_ctx *c, int k) {
     if (c->timing) cudaEventRecord(c->ev[k], c->stream);
 }
@@ -408,13 +421,7 @@ int force_pass(nbody_ctx *c, int damping, double theta, bool fp64, bool want_vma
     unsigned launches = 0;
     tree_inputs(c, n, want_vmax);
     if (pos) c->tb.pos = pos;
-    const bool multi = c->nsys > 1 && !c->single_pass && c->sys_total == n;
-    c->tb.nsys = multi ? c->nsys : 1;
-    c->tb.sys_start = c->sys_start;
-    c->tb.sys_id = c->sys_id;
-    c->tb.sys_sorted = c->sys_sorted;
-    c->tb.sys_root = c->sys_root;
-    c->tb.sys_root_node = c->sys_root_node;
+    const bool multi = tree_layout(c);
     ev(c, 0);
     if (restore_slot >= 0 && !multi) {
         // the octree of these positions was saved by the forward recomputation
@@ -781,6 +788,7 @@ int run_steps(nbody_ctx *c, uint32_t nsteps, uint32_t in_call) {
             if (capture(c, &c->step_exec, &c->step_launches, [&] { return one_step(c); })) c->step_key = key;
         }
         if (c->step_exec && key == c->step_key) {
+            tree_layout(c);  // what check_status reports of the replayed builds
             for (uint32_t s = 0; s < nsteps; s++) {
                 NB_CUDA(cudaGraphLaunch(c->step_exec, c->stream));
                 c->launches += c->step_launches;
@@ -1496,6 +1504,7 @@ int nbody_backward(nbody_ctx *c, const double *dL_dpos, const double *dL_dvel, d
     MultiStepCall scope(c, K > 1);
     int rc = begin_call(c);
     if (rc) return rc;
+    tree_layout(c);
     {
         auto key = graph_key(c, C);
         if (key != c->adj_key) {

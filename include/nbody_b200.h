@@ -162,8 +162,9 @@ typedef struct nbody_stats {
     uint64_t walk_decisions;     /* internal nodes the warps decided (open / accept) */
     uint64_t walk_list;          /* bodies the warps put in their interaction lists */
     uint64_t walk_near;          /* bodies taken with FP64 offsets (too close for FP32 offsets) */
-    uint32_t walk_warps_per_block; /* walk block shape in use (autotuned or default) */
-    uint32_t walk_blocks;          /* walk grid size in use (persistent blocks) */
+    uint32_t walk_warps_per_block; /* walk block shape in use (autotuned or default; a team's 4 while
+                                      teams of warps walk the groups of a small state) */
+    uint32_t walk_blocks;          /* walk grid size in use (persistent blocks, or the teams) */
     uint32_t tree_nodes;     /* internal nodes of the (chain-free) octree */
     uint32_t tree_depth;     /* deepest internal-node level */
     uint32_t max_stack;      /* longest queue of nodes a walk held (entries) */
@@ -207,7 +208,8 @@ int nbody_set_walk_stats(nbody_ctx *ctx, int enabled);
 int nbody_set_graphs(nbody_ctx *ctx, int enabled);
 /* Autotuner: times the walk on the resident state for each block shape (1, 2
  * or 4 warps per block, all or all-but-one resident blocks per SM) and keeps
- * the fastest for this context's precision (see nbody_stats.walk_*). */
+ * the fastest for this context's precision (see nbody_stats.walk_*). A state
+ * that teams of warps walk has one shape, and leaves the kept one alone. */
 int nbody_autotune(nbody_ctx *ctx);
 
 typedef struct nbody_diagnostics {

@@ -320,6 +320,15 @@ struct MultiStepCall {
     ~MultiStepCall() { c->multi_step_call = saved; }
 };
 
+// The groups of a forward walk of the octree last built (TreeBuild::n, nsys), and
+// whether teams walk them.
+uint32_t forward_groups(const nbody_ctx *c) { return c->tb.nsys > 1 ? c->ngroups : (c->tb.n + 31) / 32; }
+bool forward_by_teams(const nbody_ctx *c) {
+    const bool fp64 = c->p.precision == NBODY_PRECISION_FP64;
+    return walk_by_teams(fp64, false, c->tb.n, forward_groups(c), (uint32_t)std::max(1, (int)c->tb.nsys),
+                         fp64 ? c->wl_fp64 : c->wl_mixed);
+}
+
 int check_status(nbody_ctx *c) {
     NB_CUDA(cudaStreamSynchronize(c->stream));
     const DevScalars &h = *c->hsc;
@@ -334,8 +343,9 @@ int check_status(nbody_ctx *c) {
     s.kernel_launches = c->launches;
     {
         const WalkLaunch &w = c->p.precision == NBODY_PRECISION_FP64 ? c->wl_fp64 : c->wl_mixed;
-        s.walk_warps_per_block = w.warps;
-        s.walk_blocks = w.blocks;
+        const bool team = forward_by_teams(c);
+        s.walk_warps_per_block = team ? kTeamMaxWarps : w.warps;
+        s.walk_blocks = team ? team_blocks(forward_groups(c), w) : w.blocks;
     }
     s.merged_min_size = c->merged_min_size;
     s.merged_collisions = c->merged_collisions;
@@ -924,11 +934,15 @@ int adjoint_force(nbody_ctx *c, const double *pos, int damping, double theta, bo
 // per block; all or all-but-one resident blocks per SM) and keeps the fastest
 // for this context's precision. Tree and COM are rebuilt per candidate so each
 // walk starts from the same state; only the walk is timed (CUDA events, best of 3).
+// Teams have one shape: the first candidate's passes leave the forces and statistics,
+// and the shape of single warps stays what it is.
 std::vector<unsigned char> tune_key(nbody_ctx *c) {
-    struct K { uint32_t n_bucket, nsys; int precision, damping; double theta; } k;
+    struct K { uint32_t n_bucket, nsys; int precision, damping, team; double theta; } k;
     std::memset(&k, 0, sizeof k);
     uint32_t b = 1;
     while (b < c->n) b <<= 1;
+    tree_layout(c);
+    k.team = forward_by_teams(c);  // (their sizes end within a bucket)
     k.n_bucket = b; k.nsys = c->nsys; k.precision = c->p.precision; k.damping = c->p.damping; k.theta = c->p.theta;
     const unsigned char *p = (const unsigned char *)&k;
     return std::vector<unsigned char>(p, p + sizeof k);
@@ -939,6 +953,8 @@ int autotune(nbody_ctx *c) {
     const int saved_timing = c->timing;
     c->timing = 1;
     WalkLaunch best = fp64 ? c->wl_fp64 : c->wl_mixed;
+    tree_layout(c);
+    const bool team = forward_by_teams(c);
     float best_ms = 1e30f;
     int rc = NBODY_OK;
     for (unsigned w : {1u, 2u, 4u}) {
@@ -963,12 +979,13 @@ int autotune(nbody_ctx *c) {
                 ms = std::min(ms, c->stats.ms_walk);
             }
             if (rc) break;
+            if (team) break;
             if (ms < best_ms) {
                 best_ms = ms;
                 best = shape;
             }
         }
-        if (rc) break;
+        if (rc || team) break;
     }
     c->timing = saved_timing;
     if (rc) return rc;

@@ -32,6 +32,7 @@
 #include "walk.cuh"
 #include "fp64.cuh"
 
+#include <algorithm>
 #include <type_traits>
 
 namespace nbody {
@@ -1300,13 +1301,18 @@ cudaError_t walk_launch_shape(bool fp64, int device, unsigned warps, unsigned bl
     return cudaSuccess;
 }
 
+bool walk_by_teams(bool fp64, bool adjoint, uint32_t n, uint32_t n_groups, uint32_t systems, const WalkLaunch &l) {
+    return n_groups <= team_groups_per_sm(fp64, adjoint) * l.sms && n >= kTeamMinSize * systems;
+}
+
+// One block per group, as many as fit; the rest take the groups left.
+unsigned team_blocks(uint32_t n_groups, const WalkLaunch &l) { return std::min(n_groups, kTeamBlocksPerSm * l.sms); }
+
 cudaError_t launch_walk(const WalkArgs &a, bool fp64, const WalkLaunch &l, cudaStream_t st) {
     const bool adj = a.adjoint != 0;
-    const bool team = a.n_groups <= team_groups_per_sm(fp64, adj) * l.sms && a.t.n >= kTeamMinSize * a.systems;
+    const bool team = walk_by_teams(fp64, adj, a.t.n, a.n_groups, a.systems, l);
     const void *k = any_walk_kernel(team, fp64, adj, a.damping, a.pot != nullptr, a.stats != 0);
-    if (team)  // one block per group, as many as fit; the rest take the groups left
-        return launch(k, a, a.n_groups < kTeamBlocksPerSm * l.sms ? a.n_groups : kTeamBlocksPerSm * l.sms, kTeamMaxWarps,
-                      team_smem(fp64, adj), st);
+    if (team) return launch(k, a, team_blocks(a.n_groups, l), kTeamMaxWarps, team_smem(fp64, adj), st);
     const unsigned need = (a.n_groups + l.warps - 1) / l.warps;
     return launch(k, a, need < l.blocks ? need : l.blocks, l.warps, solo_smem(fp64, adj) * l.warps, st);
 }

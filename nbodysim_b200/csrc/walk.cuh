@@ -82,6 +82,9 @@ struct WalkLaunch {
 cudaError_t walk_launch_shape(bool fp64, int device, unsigned warps, unsigned blocks_per_sm, WalkLaunch *out);
 // Resident blocks per SM that fit for `warps` per block (all forward instances).
 cudaError_t walk_max_blocks_per_sm(bool fp64, unsigned warps, int *out);
+// Whether teams walk n particles in n_groups groups, and their grid (blocks of kTeamMaxWarps).
+bool walk_by_teams(bool fp64, bool adjoint, uint32_t n, uint32_t n_groups, uint32_t systems, const WalkLaunch &l);
+unsigned team_blocks(uint32_t n_groups, const WalkLaunch &l);
 cudaError_t launch_walk(const WalkArgs &a, bool fp64, const WalkLaunch &l, cudaStream_t st);
 
 }  // namespace nbody

@@ -201,7 +201,7 @@ int reserve(nbody_ctx *c, uint32_t n) {
         {(void **)&tb.sort_scratch, sort_scratch_bytes(cap)}, {(void **)&tb.scan_tmp, 4 * scan_tiles},
         {(void **)&tb.body, 32 * N}, {(void **)&tb.onode, 32 * N},
         {(void **)&tb.bleft, 4 * N}, {(void **)&tb.bright, 4 * N}, {(void **)&tb.bparent, 4 * N},
-        {(void **)&tb.leaf_bparent, 4 * N}, {(void **)&tb.bdelta, 4 * N},
+        {(void **)&tb.bdelta, 4 * N},
         {(void **)&tb.head_flag, 4 * N}, {(void **)&tb.head_id, 4 * N}, {(void **)&tb.ocount, 4 * N},
         {(void **)&tb.ochild, 32 * N}, {(void **)&tb.ometa, 4 * N}, {(void **)&tb.oparent, 4 * N},
         {(void **)&tb.leaf_oparent, 4 * N},

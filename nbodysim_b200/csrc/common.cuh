@@ -7,7 +7,7 @@
 //                 acc       : float[3*cap] (MIXED) or double[3*cap] (FP64)
 //   sort          key1/idx  : u64/u32 [cap] x2 (ping-pong), key2/key3 u64[cap] (deep keys)
 //   sorted bodies body      : double4[cap] = (x, y, z, m) in Morton order
-//   binary tree   bleft/bright/bparent : i32[cap], bdelta u8..i32[cap], leaf_bparent i32[cap]
+//   binary tree   bleft/bright/bparent : i32[cap], bdelta u8..i32[cap]
 //   octree        onode     : double4[cap] = (com.x, com.y, com.z, mass)
 //                 ochild    : i32[8*cap]  (>= 0 internal node, < 0 leaf ~sorted index)
 //                 ometa     : i32[cap]    level | nchild << 8

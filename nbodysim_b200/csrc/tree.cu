@@ -558,9 +558,8 @@ __device__ inline int radix_node(const KeyView &kv, int i, int dn, int &left, in
 }
 
 __global__ void k_radix_tree(KeyView kv, int32_t *__restrict__ bleft, int32_t *__restrict__ bright,
-                             int32_t *__restrict__ bparent, int32_t *__restrict__ leaf_bparent,
-                             int32_t *__restrict__ bdelta, uint32_t *max_prefix_bits, uint32_t *pair_passes,
-                             uint32_t sys_bits) {
+                             int32_t *__restrict__ bparent, int32_t *__restrict__ bdelta, uint32_t *max_prefix_bits,
+                             uint32_t *pair_passes, uint32_t sys_bits) {
     __shared__ uint32_t hist[kPassBins];
     griddep();
     int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -594,8 +593,8 @@ __global__ void k_radix_tree(KeyView kv, int32_t *__restrict__ bleft, int32_t *_
     bleft[i] = left;
     bright[i] = right;
     bdelta[i] = dnode;
-    if (left >= 0) bparent[left] = i; else leaf_bparent[~left] = i;
-    if (right >= 0) bparent[right] = i; else leaf_bparent[~right] = i;
+    if (left >= 0) bparent[left] = i;
+    if (right >= 0) bparent[right] = i;
     if (seg_root) bparent[i] = -1;
 }
 
@@ -1338,9 +1337,8 @@ cudaError_t build_octree(const TreeBuild &tb, cudaStream_t st, unsigned *launche
                                                        sys_sorted, tb.sys_root, tb.sc, tb.single);
     KeyView kv{tb.key_b, tb.key_a, tb.key3, (int)n, sys_sorted};
     const uint32_t m = n - 1;
-    launch_pdl(k_radix_tree, dim3(blocks_for(m, 256)), dim3(256), 0, st, kv, tb.bleft, tb.bright, tb.bparent, tb.leaf_bparent,
-                                                      tb.bdelta, &tb.sc->max_prefix_bits, tb.sc->pair_passes,
-               multi ? (uint32_t)tb.sys_bits : 0u);
+    launch_pdl(k_radix_tree, dim3(blocks_for(m, 256)), dim3(256), 0, st, kv, tb.bleft, tb.bright, tb.bparent, tb.bdelta,
+               &tb.sc->max_prefix_bits, tb.sc->pair_passes, multi ? (uint32_t)tb.sys_bits : 0u);
     launch_pdl(k_head_flags, dim3(blocks_for(n, 256)), dim3(256), 0, st, tb.bparent, tb.bdelta, m, tb.head_flag,
                tb.head_id, tb.oparent, tb.leaf_oparent, tb.ocount);
     L += 3 + scan_exclusive(tb.head_id, m, tb.scan_tmp, &tb.sc->n_onodes, st);

@@ -40,7 +40,7 @@ struct TreeBuild {
     uint32_t *sort_scratch;     // sort_scratch_bytes(n)
     uint32_t *scan_tmp;         // ceil(max_len / 4096) + 1
     double4 *body;
-    int32_t *bleft, *bright, *bparent, *leaf_bparent, *bdelta;
+    int32_t *bleft, *bright, *bparent, *bdelta;
     uint32_t *head_flag, *head_id;
     int32_t *ochild, *ometa, *oparent, *leaf_oparent;
     uint32_t *ocount;

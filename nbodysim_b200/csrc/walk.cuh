@@ -22,18 +22,27 @@ constexpr int kSoloList = 64;
 constexpr int kTeamList = 32 + 32 * kTeamMaxWarps;
 // Teams walk while there are at most this many groups per SM. Fewer groups leave
 // walk warps idle, and time is the chain of one group's tiles; with more, barriers
-// cost more than the last wave of single warps. Walk times, team against single
-// warps (us): MIXED 5000 particles 51 / 103, shell of 20,011 50 / 89, cubes of 48,000
-// 170 / 197, 56,000 195 / 206 and 70,000 240 / 228; its adjoint 5000 89 / 183, 85,000
-// 578 / 598, 100,000 682 / 648; FP64 (with the pair terms of then) 5000 135 / 375,
-// 16,384 226 / 580, 60,001 885 / 1168, 112,000 1006 / 1235; its adjoint 16,384 310 /
-// 671, 100,000 1460 / 1591.
+// cost more than the last wave of single warps. Where that is depends on the state: a
+// shell's short lists suit single warps sooner than a sphere's long ones. Walk times,
+// teams against single warps (us):
+//   MIXED: 5000 particles 51 / 96, shell of 20,011 53 / 82; 40,000: shell 94 / 101,
+//   sphere 183 / 203; 48,000: shell 115 / 100, cube 172 / 185, sphere 201 / 210,
+//   collapsed 255 / 262; 56,000: 131 / 106, 198 / 189, 231 / 218, 284 / 262.
+//   Its adjoint: 5000 95 / 175; spheres of 60,000 401 / 441, 72,000 466 / 476, 85,000
+//   536 / 537, 100,000 636 / 588.
+//   FP64: 5000 86 / 210, 16,384 147 / 322, 60,001 (damped) 788 / 950; 85,000: sphere
+//   540 / 580, shell 296 / 248; 112,000: sphere 680 / 732, collapsed 880 / 847, shell
+//   379 / 336; 150,000: sphere 900 / 887.
+//   Its adjoint: 16,384 257 / 548, 100,000 1246 / 1380, 113,000 1397 / 1453.
 // Systems of fewer than kTeamMinSize particles have a few short tiles per group, for
 // which the barriers cost more (a step of 97: 133 us with teams, 125 without; 150:
 // the same; 300: 147 and 151).
 constexpr uint32_t kTeamMinSize = 160;
-constexpr unsigned team_groups_per_sm(bool fp64, bool adjoint) { return fp64 ? 24 : adjoint ? 16 : 12; }
-constexpr unsigned kTeamBlocksPerSm = 5;  // resident: 96 registers, ~36 KB of shared memory
+constexpr unsigned team_groups_per_sm(bool fp64, bool adjoint) { return fp64 ? 24 : adjoint ? 16 : 10; }
+// Blocks per SM of a team grid: as many as are resident (at most 96 registers, 36 KB of
+// shared memory). The FP64 adjoint's take 128 and 168 registers: three or four are
+// resident, and the others start as those end and find the groups drained.
+constexpr unsigned kTeamBlocksPerSm = 5;
 
 struct WalkArgs {
     Tree t;

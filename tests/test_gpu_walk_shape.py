@@ -1,5 +1,7 @@
-"""GPU: the walk's block shape where teams of warps walk the groups: what the statistics
-report, and that tuning such a state does not choose the shape of single warps."""
+"""GPU: the walk's block shape where teams of warps walk the groups (MIXED: up to ten
+groups an SM): what the statistics report, that tuning such a state does not choose the
+shape of single warps, and the reference's counts on both sides of the limit."""
+import numpy as np
 import pytest
 import torch
 
@@ -8,7 +10,7 @@ pytestmark = pytest.mark.gpu
 
 def test_statistics_report_the_teams(nb):
     sms = torch.cuda.get_device_properties(0).multi_processor_count
-    for n, team in ((100, False), (5000, True), (50001, True)):
+    for n, team in ((100, False), (5000, True), (40001, True), (320 * sms, True), (320 * sms + 1, False), (50001, False)):
         pos, vel, mass = nb.generate(n, gen_type=1, seed=1)
         with nb.Engine() as e:
             e.set_particles(pos, vel, mass)
@@ -21,7 +23,7 @@ def test_statistics_report_the_teams(nb):
 
 def test_a_state_for_single_warps_is_tuned_after_one_for_teams(nb):
     """Both sizes lie in one power of two."""
-    limit = 12 * 32 * torch.cuda.get_device_properties(0).multi_processor_count
+    limit = 10 * 32 * torch.cuda.get_device_properties(0).multi_processor_count
     spent = []
     with nb.Engine(autotune=1) as e:
         for n in (limit - 500, limit + 500):
@@ -33,3 +35,18 @@ def test_a_state_for_single_warps_is_tuned_after_one_for_teams(nb):
         assert e.stats()["walk_warps_per_block"] in (1, 2, 4)
     # 3 passes and a step; 3 passes for each of up to 6 shapes and a step
     assert spent[1] > 2 * spent[0]
+
+
+@pytest.mark.parametrize("more", [0, 1])
+def test_counts_on_both_sides_of_the_mixed_limit(nb, orc, more):
+    n = 10 * 32 * torch.cuda.get_device_properties(0).multi_processor_count + more
+    pos, vel, mass = nb.generate(n, gen_type=2, size=1024.0, seed=n)
+    sample = np.sort(np.random.default_rng(n).choice(n, 300, replace=False)).astype(np.uint32)
+    sample[-1] = n - 1
+    with nb.Engine() as e:
+        acc, cnt = e.barnes_hut(pos, mass, counts=True)
+        assert (e.stats()["walk_blocks"] == 5 * torch.cuda.get_device_properties(0).multi_processor_count) == (more == 0)
+    ref, want = orc.forces(pos, mass, 0.5, sample=sample)
+    assert np.array_equal(cnt[sample], want)
+    err = np.linalg.norm(acc[sample] - ref, axis=1) / np.linalg.norm(ref, axis=1)
+    assert np.percentile(err, 99) <= 1e-5

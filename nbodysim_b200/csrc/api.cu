@@ -325,7 +325,7 @@ struct MultiStepCall {
 uint32_t forward_groups(const nbody_ctx *c) { return c->tb.nsys > 1 ? c->ngroups : (c->tb.n + 31) / 32; }
 bool forward_by_teams(const nbody_ctx *c) {
     const bool fp64 = c->p.precision == NBODY_PRECISION_FP64;
-    return walk_by_teams(fp64, false, c->tb.n, forward_groups(c), (uint32_t)std::max(1, (int)c->tb.nsys),
+    return walk_by_teams(fp64, false, c->p.theta, c->tb.n, forward_groups(c), (uint32_t)std::max(1, (int)c->tb.nsys),
                          fp64 ? c->wl_fp64 : c->wl_mixed);
 }
 
@@ -472,6 +472,7 @@ int force_pass(nbody_ctx *c, int damping, double theta, bool fp64, bool want_vma
     a.counts = want_counts ? c->counts : nullptr;
     a.pot = want_pot ? c->pot : nullptr;
     a.queue = c->queue;
+    a.wide = queue_wide(theta);
     a.n_groups = multi ? c->ngroups : (n + 31) / 32;
     a.systems = multi ? c->nsys : 1;
     a.groups = multi ? c->groups : nullptr;

@@ -581,13 +581,13 @@ __device__ inline void sum_batch(G &s, int start, int count, int lane, const Wal
 // The walk of one group of up to 32 particles, by one warp (kTeam false) or by the
 // warps of a block together (kTeam true).
 //
-// Both do the same arithmetic in the same order. The entries still to be examined
-// wait in a queue, first in first out, so the sequence in which they are examined,
-// and with it the sequence of every interaction list, does not depend on how many
-// are examined at a time; each list is summed in batches of 32 consecutive entries,
-// the batches' sums are added in order, and the lists' sums last. (Past kQueueWide
-// waiting entries the newest go first, one tile at a time, which bounds the queue;
-// a team takes no more tiles at once than keep the order of one warp's walk.)
+// Both do the same arithmetic in the same order. The entries still to be examined wait
+// in a queue, which is taken in batches of a team's four tiles. Which entries come next
+// (walk.cuh) is decided when a batch is done, and children queue up in the order of their
+// parents, so the sequence in which entries are examined, and with it the sequence of
+// every interaction list, does not depend on how many are examined at a time. Each list
+// is summed in batches of 32 consecutive entries, the batches' sums are added in order,
+// and the lists' sums last.
 //
 // Nodes, bodies and children are gathered, one 32-byte load each. Many groups keep the
 // load pipe of the L1 and shared memory at 76% beside 69% of the issue slots (1M bodies,
@@ -742,27 +742,40 @@ __global__ void __launch_bounds__((kTeam ? kTeamMaxWarps : kWalkMaxWarps) * 32) 
         uint32_t cnt = 0, nint = 0, nfallback = 0;
         uint32_t head = 0, qn = root >= 0 ? 1u : 0u;       // the queue: first entry, entries
         uint32_t lstart[3] = {0, 0, 0}, lcount[3] = {0, 0, 0};  // each list's ring: first entry, entries
-        // the next tile's entries, loaded a tile early where the queue (in global memory)
-        // holds them all already: -1 to -2% walk time
+        // One warp examines a batch tile by tile: the tiles still to come (they are at the
+        // queue's front), and the tile's entries, which are loaded a tile early where the
+        // queue (in global memory) holds them all already (else their masks are 0).
+        uint32_t left = 0;
         int2 ahead = make_int2(0, 0);
-        bool have_ahead = false;
         sync();
 
         while (qn > 0) {
-            uint32_t base, take;
-            if (qn <= kQueueWide) {
-                // a team takes whole tiles, as many as cannot take the queue past kQueueWide
-                // between them (one warp would turn to the newest entries there)
-                const uint32_t tiles = kTeam ? max(1u, min(min(W, qn / 32u), 1u + (kQueueWide - qn) / 224u)) : 1u;
-                base = head;
-                take = min(qn, 32u * tiles);
-                head += take;
+            uint32_t base = head, take = 32;
+            if (!kTeam && left > 0) {
+                left--;
+                head += 32;
             } else {
-                // the newest entries; fewer as the queue fills, down to a depth-first
-                // descent of one at a time, for which kQueueReserve is room
-                const int room = ((int)(kQueueCap - kQueueReserve) - (int)qn) / 8;
-                take = (uint32_t)max(1, min(32, room));
-                base = head + qn - take;
+                const bool newest = qn > a.wide;
+                take = min(qn, kQueueBatch);
+                if (newest) {
+                    const int room = ((int)(kQueueCap - kQueueReserve) - (int)qn) / 8;
+                    take = (uint32_t)max(1, min(room, (int)kQueueBatch));
+                }
+                if (take > 32u) take &= ~31u;
+                if (newest) base = head + qn - take;
+                else head += kTeam ? take : min(take, 32u);
+                if constexpr (!kTeam) {
+                    left = (take - 1u) / 32u;
+                    if (newest) {
+                        // the other tiles move to the front, as children take their place
+                        for (uint32_t q = 32u + lane; q < take; q += 32u)
+                            queue[(head - take + q) & (kQueueCap - 1)] = queue[(base + q) & (kQueueCap - 1)];
+                        head -= 32u * left;
+                    }
+                    take = min(take, 32u);
+                    if (newest || ahead.y == 0) ahead = queue[(base + min((uint32_t)lane, take - 1u)) & (kQueueCap - 1)];
+                    __syncwarp();  // all read before any lane writes there
+                }
             }
             qn -= take;
             const int cntt = take > 32u * w ? (int)min(32u, take - 32u * w) : 0;
@@ -778,9 +791,7 @@ __global__ void __launch_bounds__((kTeam ? kTeamMaxWarps : kWalkMaxWarps) * 32) 
             int nch = 0, ref = 0;
             double cx = 0, cy = 0, cz = 0, m = 0, so = 0;
             if (lane < cntt) {
-                const int2 e = !kTeam && have_ahead && base == head - 32u
-                                   ? ahead
-                                   : queue[(base + 32u * w + lane) & (kQueueCap - 1)];
+                const int2 e = kTeam ? queue[(base + 32u * w + lane) & (kQueueCap - 1)] : ahead;
                 ref = e.x;
                 reach = (uint32_t)e.y;
                 if (ref >= 0) {
@@ -798,10 +809,7 @@ __global__ void __launch_bounds__((kTeam ? kTeamMaxWarps : kWalkMaxWarps) * 32) 
                     if (own < 32u) reach &= ~(1u << own);
                 }
             }
-            if constexpr (!kTeam) {
-                have_ahead = qn >= 32u;
-                if (have_ahead) ahead = queue[(head + lane) & (kQueueCap - 1)];
-            }
+            if constexpr (!kTeam) ahead = qn >= 32u ? queue[(head + lane) & (kQueueCap - 1)] : make_int2(0, 0);
             float fcx = 0.f, fcy = 0.f, fcz = 0.f;
             if constexpr (!kFp64) {
                 fcx = (float)(cx - s.gc.ref[0]); fcy = (float)(cy - s.gc.ref[1]); fcz = (float)(cz - s.gc.ref[2]);
@@ -1301,8 +1309,9 @@ cudaError_t walk_launch_shape(bool fp64, int device, unsigned warps, unsigned bl
     return cudaSuccess;
 }
 
-bool walk_by_teams(bool fp64, bool adjoint, uint32_t n, uint32_t n_groups, uint32_t systems, const WalkLaunch &l) {
-    return n_groups <= team_groups_per_sm(fp64, adjoint) * l.sms && n >= kTeamMinSize * systems;
+bool walk_by_teams(bool fp64, bool adjoint, double theta, uint32_t n, uint32_t n_groups, uint32_t systems,
+                   const WalkLaunch &l) {
+    return n_groups <= team_groups_per_sm(fp64, adjoint, theta) * l.sms && n >= kTeamMinSize * systems;
 }
 
 // One block per group, as many as fit; the rest take the groups left.
@@ -1310,7 +1319,7 @@ unsigned team_blocks(uint32_t n_groups, const WalkLaunch &l) { return std::min(n
 
 cudaError_t launch_walk(const WalkArgs &a, bool fp64, const WalkLaunch &l, cudaStream_t st) {
     const bool adj = a.adjoint != 0;
-    const bool team = walk_by_teams(fp64, adj, a.t.n, a.n_groups, a.systems, l);
+    const bool team = walk_by_teams(fp64, adj, a.theta, a.t.n, a.n_groups, a.systems, l);
     const void *k = any_walk_kernel(team, fp64, adj, a.damping, a.pot != nullptr, a.stats != 0);
     if (team) return launch(k, a, team_blocks(a.n_groups, l), kTeamMaxWarps, team_smem(fp64, adj), st);
     const unsigned need = (a.n_groups + l.warps - 1) / l.warps;

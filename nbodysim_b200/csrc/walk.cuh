@@ -8,15 +8,28 @@ namespace nbody {
 constexpr int kWalkWarps = 4;       // default warps per block (the autotuner may pick 1 or 2)
 constexpr int kWalkMaxWarps = 4;    // largest block the walk kernel is compiled for
 constexpr int kTeamMaxWarps = 4;    // warps of a block that walk one group together
-// Queue of the nodes a walk has still to examine (per warp in global memory, per
-// team in shared memory). Up to kQueueWide entries the oldest go first; beyond, the
-// newest, in tiles that get narrower until a depth-first descent of one entry at a
-// time (at most 7 more entries per level) fits in the reserve.
+// Queue of the nodes a walk has still to examine (per warp in global memory, per team
+// in shared memory), taken in batches of kQueueBatch: a team's turn. While no more than
+// queue_wide(theta) wait, the oldest go first; beyond, the newest, in batches that get
+// smaller until a depth-first descent of one entry at a time (at most 7 more entries per
+// level) fits in the reserve.
+//
+// Oldest first keeps tiles full and reads nodes level by level; newest first bounds the
+// queue. A small opening angle opens so many nodes that the queue is at its limit for most
+// of the walk, and a low one leaves room for whole batches (MIXED cube / sphere of 20,000,
+// us: theta 0.1 limit 256: 868 / 789, 640: 1356 / 1108; 0.3: 195 / 205 and 231 / 268;
+// 0.5: 82 / 90 both). At ordinary angles few walks pass 640 (collapsed system of 1,048,576:
+// 3530 with 256, 3468 with 640). One tile at a time past 1280 left a team's other warps
+// idle and made tiles narrow: 40,000 at theta 0.05 8.9 ms, at 0.3 0.75, now 3.7 and 0.41.
 constexpr uint32_t kQueueCap = 2048;
-constexpr uint32_t kQueueWide = 1280;
+constexpr uint32_t kQueueWide = 640, kQueueWideSmallTheta = 256;
+constexpr uint32_t queue_wide(double theta) { return theta < 0.45 ? kQueueWideSmallTheta : kQueueWide; }
+constexpr uint32_t kQueueBatch = 32 * kTeamMaxWarps;
 constexpr uint32_t kQueueReserve = 7 * (kMaxLevels + 1) + 8;
 static_assert((kQueueCap & (kQueueCap - 1)) == 0, "ring index");
-static_assert(kQueueWide + 8 * 32 <= kQueueCap - kQueueReserve, "a tile's pushes fit before tiles get narrower");
+static_assert(kQueueWide + 7 * kQueueBatch <= kQueueCap - kQueueReserve, "a batch's pushes fit before batches get smaller");
+static_assert(kQueueWideSmallTheta >= kQueueBatch && kQueueWide >= kQueueBatch, "past the limit there is a whole batch");
+static_assert(kQueueBatch <= kQueueReserve, "room for a batch moved to the front");
 // Interaction lists: less than a batch of 32 left over, and what a tile (a team's tiles) adds.
 constexpr int kSoloList = 64;
 constexpr int kTeamList = 32 + 32 * kTeamMaxWarps;
@@ -38,7 +51,9 @@ constexpr int kTeamList = 32 + 32 * kTeamMaxWarps;
 // which the barriers cost more (a step of 97: 133 us with teams, 125 without; 150:
 // the same; 300: 147 and 151).
 constexpr uint32_t kTeamMinSize = 160;
-constexpr unsigned team_groups_per_sm(bool fp64, bool adjoint) { return fp64 ? 24 : adjoint ? 16 : 10; }
+constexpr unsigned team_groups_per_sm(bool fp64, bool adjoint, double theta) {
+    return fp64 ? 24 : adjoint ? 16 : theta < 0.25 ? 7 : 10;
+}
 // Blocks per SM of a team grid: as many as are resident (at most 96 registers, 36 KB of
 // shared memory). The FP64 adjoint's take 128 and 168 registers: three or four are
 // resident, and the others start as those end and find the groups drained.
@@ -56,6 +71,7 @@ struct WalkArgs {
     uint32_t *counts;   // optional: accepted nodes per particle (user order)
     double *pot;        // optional: potential phi_i per particle (user order)
     int2 *queue;        // kQueueCap entries per warp of the grid (walks by one warp)
+    uint32_t wide;      // queue_wide(theta)
     uint32_t n_groups;  // ceil(n / 32)
     uint32_t systems;   // independent systems (1: a single one)
     int track_max_acc;  // reduce max |a| (adaptive dt)
@@ -92,7 +108,8 @@ cudaError_t walk_launch_shape(bool fp64, int device, unsigned warps, unsigned bl
 // Resident blocks per SM that fit for `warps` per block (all forward instances).
 cudaError_t walk_max_blocks_per_sm(bool fp64, unsigned warps, int *out);
 // Whether teams walk n particles in n_groups groups, and their grid (blocks of kTeamMaxWarps).
-bool walk_by_teams(bool fp64, bool adjoint, uint32_t n, uint32_t n_groups, uint32_t systems, const WalkLaunch &l);
+bool walk_by_teams(bool fp64, bool adjoint, double theta, uint32_t n, uint32_t n_groups, uint32_t systems,
+                   const WalkLaunch &l);
 unsigned team_blocks(uint32_t n_groups, const WalkLaunch &l);
 cudaError_t launch_walk(const WalkArgs &a, bool fp64, const WalkLaunch &l, cudaStream_t st);
 

@@ -103,6 +103,7 @@ struct nbody_ctx {
     double *sys_root = nullptr;
     int32_t *sys_root_node = nullptr;
     bool single_pass = false;  // nbody_barnes_hut: one system regardless of the layout
+    double pass_theta = 0.5;   // of the last force pass
     // Sort plan of the next tree build (TreeBuild::sort_p1, sort_p2): the full
     // two-word sort until a build has measured its pairs of neighbours, then the
     // passes next_sort_plan picks from them. The build sorts the runs of
@@ -325,7 +326,7 @@ struct MultiStepCall {
 uint32_t forward_groups(const nbody_ctx *c) { return c->tb.nsys > 1 ? c->ngroups : (c->tb.n + 31) / 32; }
 bool forward_by_teams(const nbody_ctx *c) {
     const bool fp64 = c->p.precision == NBODY_PRECISION_FP64;
-    return walk_by_teams(fp64, false, c->p.theta, c->tb.n, forward_groups(c), (uint32_t)std::max(1, (int)c->tb.nsys),
+    return walk_by_teams(fp64, false, c->pass_theta, c->tb.n, forward_groups(c), (uint32_t)std::max(1, (int)c->tb.nsys),
                          fp64 ? c->wl_fp64 : c->wl_mixed);
 }
 
@@ -402,8 +403,9 @@ void tree_inputs(nbody_ctx *c, uint32_t n, bool want_vmax) {
     tb.reset = 0;
 }
 
-// The systems that a force pass on the state takes it for; true if there are several.
-bool tree_layout(nbody_ctx *c) {
+// The systems that a force pass at `theta` on the state takes it for; true if there are several.
+bool tree_layout(nbody_ctx *c, double theta) {
+    c->pass_theta = theta;
     const bool multi = c->nsys > 1 && !c->single_pass && c->sys_total == c->n;
     c->tb.n = c->n;
     c->tb.nsys = multi ? c->nsys : 1;
@@ -431,7 +433,7 @@ int force_pass(nbody_ctx *c, int damping, double theta, bool fp64, bool want_vma
     unsigned launches = 0;
     tree_inputs(c, n, want_vmax);
     if (pos) c->tb.pos = pos;
-    const bool multi = tree_layout(c);
+    const bool multi = tree_layout(c, theta);
     ev(c, 0);
     if (restore_slot >= 0 && !multi) {
         // the octree of these positions was saved by the forward recomputation
@@ -799,7 +801,7 @@ int run_steps(nbody_ctx *c, uint32_t nsteps, uint32_t in_call) {
             if (capture(c, &c->step_exec, &c->step_launches, [&] { return one_step(c); })) c->step_key = key;
         }
         if (c->step_exec && key == c->step_key) {
-            tree_layout(c);  // what check_status reports of the replayed builds
+            tree_layout(c, c->p.theta);  // what check_status reports of the replayed builds
             for (uint32_t s = 0; s < nsteps; s++) {
                 NB_CUDA(cudaGraphLaunch(c->step_exec, c->stream));
                 c->launches += c->step_launches;
@@ -942,7 +944,7 @@ std::vector<unsigned char> tune_key(nbody_ctx *c) {
     std::memset(&k, 0, sizeof k);
     uint32_t b = 1;
     while (b < c->n) b <<= 1;
-    tree_layout(c);
+    tree_layout(c, c->p.theta);
     k.team = forward_by_teams(c);  // (their sizes end within a bucket)
     k.n_bucket = b; k.nsys = c->nsys; k.precision = c->p.precision; k.damping = c->p.damping; k.theta = c->p.theta;
     const unsigned char *p = (const unsigned char *)&k;
@@ -954,7 +956,7 @@ int autotune(nbody_ctx *c) {
     const int saved_timing = c->timing;
     c->timing = 1;
     WalkLaunch best = fp64 ? c->wl_fp64 : c->wl_mixed;
-    tree_layout(c);
+    tree_layout(c, c->p.theta);
     const bool team = forward_by_teams(c);
     float best_ms = 1e30f;
     int rc = NBODY_OK;
@@ -1522,7 +1524,7 @@ int nbody_backward(nbody_ctx *c, const double *dL_dpos, const double *dL_dvel, d
     MultiStepCall scope(c, K > 1);
     int rc = begin_call(c);
     if (rc) return rc;
-    tree_layout(c);
+    tree_layout(c, c->p.theta);
     {
         auto key = graph_key(c, C);
         if (key != c->adj_key) {

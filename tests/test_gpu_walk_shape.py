@@ -50,3 +50,16 @@ def test_counts_on_both_sides_of_the_mixed_limit(nb, orc, more):
     assert np.array_equal(cnt[sample], want)
     err = np.linalg.norm(acc[sample] - ref, axis=1) / np.linalg.norm(ref, axis=1)
     assert np.percentile(err, 99) <= 1e-5
+
+
+@pytest.mark.parametrize("theta,team", [(0.24, False), (0.25, True), (0.5, True)])
+def test_small_opening_angles_end_teams_sooner(nb, theta, team):
+    """From seven groups an SM, below 0.25; a call's own angle counts."""
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    n = 7 * 32 * sms + 1
+    pos, vel, mass = nb.generate(n, gen_type=2, size=1024.0, seed=1)
+    with nb.Engine() as e:
+        e.barnes_hut(pos, mass, theta=theta)
+        assert (e.stats()["walk_blocks"] == 5 * sms) == team
+        e.barnes_hut(pos[:-1], mass[:-1], theta=theta)
+        assert e.stats()["walk_blocks"] == 5 * sms

@@ -665,7 +665,7 @@ __device__ inline void collapse_node(int i, int L, const int32_t *bleft, const i
         // strictly downwards and stay within the level's 3 key bits, so the walk is
         // at most 3 binary nodes deep: unrolled, with nothing in local memory.
         const int c1[2] = {bleft[i], bright[i]};
-    #pragma unroll
+#pragma unroll
         for (int a = 0; a < 2; a++) {
             const int x = c1[a];
             if (!same_level(x)) {
@@ -673,7 +673,7 @@ __device__ inline void collapse_node(int i, int L, const int32_t *bleft, const i
                 continue;
             }
             const int c2[2] = {bleft[x], bright[x]};
-    #pragma unroll
+#pragma unroll
             for (int b = 0; b < 2; b++) {
                 const int y = c2[b];
                 if (!same_level(y)) {
@@ -681,7 +681,7 @@ __device__ inline void collapse_node(int i, int L, const int32_t *bleft, const i
                     continue;
                 }
                 const int c3[2] = {bleft[y], bright[y]};
-    #pragma unroll
+#pragma unroll
                 for (int c = 0; c < 2; c++) {
                     if (same_level(c3[c])) atomicOr(status, kStatusCapacity);  // deeper than 3: malformed
                     else emit(c3[c]);
@@ -803,8 +803,8 @@ __device__ inline double4 node_com(int L, int nch, Child &&child, BodyAt &&body_
     return out;
 }
 
-template <typename T>
 // (launch bounds: 4 resident blocks of 256 threads, 64 registers)
+template <typename T>
 __global__ void __launch_bounds__(256, 4)
     k_com(const double4 *__restrict__ body, const int32_t *__restrict__ oparent, const int32_t *__restrict__ ochild,
           const int32_t *__restrict__ ometa, double4 *onode, uint32_t *ocount, uint32_t n, DevScalars *sc) {
@@ -984,8 +984,8 @@ __global__ void __launch_bounds__(256)
 //
 // Bound of the general chain at these sizes: the latency of a dozen dependent
 // kernels (3 to 6 us each, whatever they do). A step of 97 particles takes 84 us
-// against 107 with the chain, of 600 109 against 134, of 1000 121 against 137. One thread per particle keeps every phase one pass; 1024 is the
-// largest block.
+// against 107 with the chain, of 600 109 against 134, of 1000 121 against 137. One
+// thread per particle keeps every phase one pass; 1024 is the largest block.
 struct SmallTree {
     uint64_t k1[kSmallTree], k2[kSmallTree], k3[kSmallTree];
     double4 body[kSmallTree], node[kSmallTree];

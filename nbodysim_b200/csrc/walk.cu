@@ -593,7 +593,8 @@ __device__ inline void sum_batch(G &s, int start, int count, int lane, const Wal
 // load pipe of the L1 and shared memory at 76% beside 69% of the issue slots (1M bodies,
 // with two 16-byte loads each), so there a node's children are loaded once it is known
 // that it is opened, as about one in three is: 981 to 946 us, and 931 with 32-byte loads;
-// a collapsed system 3585 to 3470 and 3415. The other forms wait for their loads instead
+// a collapsed system 3585 to 3470 and 3415 (945 and 3460 since the queue is taken in
+// batches, which small opening angles need). The other forms wait for their loads instead
 // (teams) or have too few warps an SM to cover a second one (FP64, adjoint) and take the
 // children along with the node (20,011 bodies: 53 us, 56 with the later load; FP64 of
 // 200,000: 1117, 1150; adjoint of 100,000: 629, 693).

@@ -38,15 +38,17 @@ constexpr int kTeamList = 32 + 32 * kTeamMaxWarps;
 // cost more than the last wave of single warps. Where that is depends on the state: a
 // shell's short lists suit single warps sooner than a sphere's long ones. Walk times,
 // teams against single warps (us):
-//   MIXED: 5000 particles 51 / 96, shell of 20,011 53 / 82; 40,000: shell 94 / 101,
-//   sphere 183 / 203; 48,000: shell 115 / 100, cube 172 / 185, sphere 201 / 210,
-//   collapsed 255 / 262; 56,000: 131 / 106, 198 / 189, 231 / 218, 284 / 262.
-//   Its adjoint: 5000 95 / 175; spheres of 60,000 401 / 441, 72,000 466 / 476, 85,000
-//   536 / 537, 100,000 636 / 588.
-//   FP64: 5000 86 / 210, 16,384 147 / 322, 60,001 (damped) 788 / 950; 85,000: sphere
-//   540 / 580, shell 296 / 248; 112,000: sphere 680 / 732, collapsed 880 / 847, shell
-//   379 / 336; 150,000: sphere 900 / 887.
-//   Its adjoint: 16,384 257 / 548, 100,000 1246 / 1380, 113,000 1397 / 1453.
+//   MIXED: 5000 particles 51 / 98, shell of 20,011 53 / 82; 40,000: shell 90 / 100,
+//   sphere 168 / 203; 48,000: shell 113 / 100, cube 162 / 186, sphere 188 / 215,
+//   collapsed 244 / 268; 56,000: 127 / 104, 190 / 195, 219 / 225, 274 / 266. Below a
+//   theta of 0.25 the teams' second wave costs more, at 0.1: 25,000 cube 1165 / 1540,
+//   sphere 1231 / 1619; 35,000: 2019 / 1955, 1942 / 2060; 40,000: 2412 / 2186, 2237 / 2293.
+//   Its adjoint: 5000 94 / 172; spheres of 60,000 381 / 414, 72,000 455 / 461, 85,000
+//   532 / 524, 100,000 606 / 582.
+//   FP64: 5000 94 / 225, 16,384 139 / 315, 60,001 (damped) 743 / 920; 85,000: sphere
+//   532 / 567, shell 293 / 242; 112,000: sphere 657 / 707, collapsed 858 / 836, shell
+//   375 / 326; 150,000: sphere 870 / 881.
+//   Its adjoint: 16,384 242 / 547, 100,000 1196 / 1380, 113,000 1346 / 1448.
 // Systems of fewer than kTeamMinSize particles have a few short tiles per group, for
 // which the barriers cost more (a step of 97: 133 us with teams, 125 without; 150:
 // the same; 300: 147 and 151).

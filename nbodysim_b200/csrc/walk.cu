@@ -389,8 +389,9 @@ __device__ inline void scatter_adj8(double *adj_node, double *adj_leaf, const in
 //
 // Bound: instruction issue, most of it these terms and the reduction (125 a chunk).
 // Packed terms: adjoint walk of 65,536 bodies 470 to 435 us, 100,000 633 to 582,
-// 500,000 2600 to 2300 (5000, where a team waits for one group's chain: 90 to 92;
-// damped 65,536, whose terms are the scalar ones as before: 880 and 894).
+// 500,000 2600 to 2300 (5000, where a team waits for one group's chain: 90 to 92).
+// Damped terms are scalar, but read the same pairs: with entries of four floats 65,536
+// takes 884 us instead of 893 and 5000 164 instead of 160.
 template <bool kDamp>
 __device__ inline void adj_list_f32(float *l, uint32_t *lm, const int *lr, int count, int lane, float px, float py,
                                     float pz, float lax, float lay, float laz, float &gx, float &gy, float &gz,
@@ -508,7 +509,8 @@ __device__ inline void adj_list_f64(const double4 *lc, const uint32_t *lm, const
 // divide per pair (and per opening test of a mixed node) were most of the walk; the
 // corrected inverse roots (fp64.cuh) and the test on squares take 16,384 particles from
 // 227 to 147 us, 200,000 from 1750 to 1107, 60,001 damped (which keeps a divide and an
-// exponential) from 890 to 790, the adjoint of 16,384 from 302 to 255.
+// exponential) from 890 to 790, the adjoint of 16,384 from 302 to 255 (139, 1092,
+// 745 and 245 since the queue is taken in batches).
 template <bool kDamp, bool kPot>
 __device__ inline void force_list_f64(const double4 *lc, const uint32_t *lm, int count, int lane, double bx,
                                       double by, double bz, double &ax, double &ay, double &az, double &pot) {
